@@ -550,7 +550,7 @@ def main():
         # ~128 tokens the matmul is still bound by the packed weight bytes (2 * batch / 0.5625 FLOP per byte against a
         # machine balance of ~250), so the roofline stays the HBM one; the tensor throughput is reported beside it.
         tf = ksum_f / ksum_t / 1e6
-        roofline.update({"kernel": "gemm_tc_kernel (+ to_half_kernel, splitk_reduce_kernel)", "traffic": None, "traffic_source": None,
+        roofline.update({"kernel": "gemm_tc_kernel (+ to_half_kernel)", "traffic": None, "traffic_source": None,
                          "tensor_TFLOPs": round(tf, 1), "tensor_peak_TFLOPs": peak_tf, "tensor_frac": round(tf / peak_tf, 4)})
         if batch >= 128:
             roofline.update({"bound": "tensor", "achieved": round(tf, 1), "peak": peak_tf, "unit": "TFLOP/s", "frac": round(tf / peak_tf, 4)})

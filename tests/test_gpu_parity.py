@@ -100,6 +100,19 @@ def test_matmul_tensor_core(pkg, name, rows, cols, tokens):
     assert np.abs(y - ref).max() <= 1e-3 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("name,rows,cols,tokens", [("q4_k", 12288, 4096, 16), ("q8_0", 4096, 11008, 40), ("q6_k", 19205, 512, 70), ("q6_k", 4100, 2048, 257),
+                                                   ("q4_k", 22016, 1024, 130), ("q8_0", 256, 256, 520), ("q4_k", 64, 5632, 513), ("q6_k", 2048, 14336, 33)])
+def test_matmul_cut_tiles_and_token_tiles(pkg, name, rows, cols, tokens):
+    """Tiles cut along K (with and without whole waves before them, one and two parts per CTA), one and several token tiles with a
+    ragged last one, one and two accumulators, rows that end inside a tile. Tolerance as above: fp16 operands."""
+    typ = TYPES[name]
+    blocks = pkg.synth.quantize(typ, pkg.synth.fill_normal(rows * cols, 13, rows + typ, 0.02))
+    x = pkg.synth.fill_normal(tokens * cols, 14, cols, 1.0).reshape(tokens, cols)
+    ref = x.astype(np.float64) @ ol.dequant("oracle", typ, blocks).reshape(rows, cols).astype(np.float64).T
+    y = pkg.api.matmul(typ, blocks, rows, cols, x)
+    assert np.abs(y - ref).max() <= 1e-3 * np.abs(ref).max()
+
+
 def test_matvec_batch_and_edge_values(pkg):
     rows, cols = 8, 512
     w = pkg.synth.fill_normal(rows * cols, 5, 9, 0.02)

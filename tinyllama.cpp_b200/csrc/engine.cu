@@ -310,6 +310,22 @@ static int launch_gemv(const b200_engine* e, GemvParams p, int batch, cudaStream
 }
 
 
+// A launch that may start while the one before it runs (the kernel waits for it with griddepcontrol.wait).
+template <typename... P, typename... A>
+static void launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  CK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
 // Starts the tensor-core matmul for T tokens (gemm_tc.cuh). x16: [T][K] fp16 activations.
 static void encode_map(CUtensorMap* tm, CUtensorMapDataType dt, int rank, const void* base, const cuuint64_t* gdim, const cuuint64_t* gstr,
                        const cuuint32_t* box, CUtensorMapSwizzle swz) {
@@ -323,39 +339,25 @@ static void launch_gemm_tc(const b200_engine* e, TcParams p, cudaStream_t st) {
   set_gemv_attrs();
   const GemvGeom g0 = gemv_geometry(p.seg[0].type, p.K);
   p.nblk = g0.nblk; p.nslab = g0.nslab; p.S = g0.S; p.S_last = g0.S_last; p.R = g0.R;
-  int ub_max0 = 0;
-  for (int s = 0; s < p.nseg; ++s) ub_max0 = std::max(ub_max0, gemv_unit_bytes(p.seg[s].type));
-  // token tile: the whole batch when it fits (two MMA halves above 256 tokens: the tile then needs a multiple of 64,
-  // and its 64 KB activation stages leave room for one stage of packed units only if those are Q4_K), else tiles of 256
-  int NT = (p.T + 31) / 32 * 32;
-  if (NT > 256) {
-    NT = (p.T + 63) / 64 * 64;
-    if (NT > TC_MAX_N) NT = TC_MAX_N;
-    if (tc_smem_bytes(NT, 4, 2, 1, (TC_M * ub_max0 + 127) / 128 * 128, p.nslab) > (size_t)TC_SMEM_MAX) NT = 256;
-  }
-  p.NT = NT;
-  p.tmem_cols = 32;
-  while (p.tmem_cols < NT) p.tmem_cols *= 2;
-  p.ntiles_m = 0;
-  int ub_max = 0;
+  const int tiles_n0 = (p.T + TC_MAX_N - 1) / TC_MAX_N;
+  p.NT = ((p.T + tiles_n0 - 1) / tiles_n0 + 31) / 32 * 32;  // token tiles of equal width
+  p.tiles_n = (p.T + p.NT - 1) / p.NT;
+  int tiles_m = 0, ub_max = 0;
   for (int s = 0; s < p.nseg; ++s) {
-    p.ntiles_m += (p.seg[s].rows + TC_M - 1) / TC_M;
+    tiles_m += (p.seg[s].rows + TC_M - 1) / TC_M;
     ub_max = std::max(ub_max, gemv_unit_bytes(p.seg[s].type));
   }
   p.error_flag = e->d_error;
-  if (p.ksplit < 1) { p.ksplit = 1; p.kblocks = p.K / 256; }
-  // shared memory: a weight-tile ring two blocks deep when the token tile is narrow enough, fewer
-  // activation stages for the widest token tiles, the rest for the packed-weight ring
+  p.ws = e->d_tc_part;
+  p.tickets = e->d_tc_tickets;
+  const TcPlan plan = tc_plan(tiles_m * p.tiles_n, p.nblk, p.NT, e->num_sms, p.ws != nullptr);
+  p.rem = plan.rem; p.ge = plan.ge; p.full = plan.full;
+  // shared memory: 128 KB of activation stages for the widest token tiles (four steps ahead), eight stages for narrow ones; the
+  // rest for packed units, whose trip from HBM the kernel lives on when there are few tokens
   p.w_stage_bytes = (TC_M * ub_max + 127) / 128 * 128;
-  static const int a_force = [] { const char* v = std::getenv("B200_TC_A_STAGES"); return v ? atoi(v) : 0; }();
-  p.a_stages = NT <= 128 ? 8 : 4;
-  if (a_force == 4 || a_force == 8) p.a_stages = a_force;
-  p.b_stages = NT > 256 ? 2 : NT > 128 ? 3 : 4;
-  auto fits = [&](int w) { return tc_smem_bytes(NT, p.a_stages, p.b_stages, w, p.w_stage_bytes, p.nslab) <= (size_t)TC_SMEM_MAX; };
-  if (p.a_stages == 8 && !fits(2)) { p.b_stages = 2; if (!fits(1)) { p.a_stages = 4; p.b_stages = NT > 256 ? 2 : NT > 128 ? 3 : 4; } }
+  p.b_stages = p.NT > 192 ? 4 : p.NT > 128 ? 5 : p.NT > 64 ? 6 : TC_B_STAGES;
   p.w_stages = TC_W_STAGES;
-  while (p.w_stages > 1 && !fits(p.w_stages)) --p.w_stages;
-  if (!fits(p.w_stages)) throw std::runtime_error("tensor-core matmul: tile does not fit shared memory");
+  while (p.w_stages > 1 && tc_smem_bytes(p.NT, p.b_stages, p.w_stages, p.w_stage_bytes) > (size_t)TC_SMEM_MAX) --p.w_stages;
   static const bool force_rowcopy = [] { const char* v = std::getenv("B200_TC_ROWCOPY"); return v && v[0] == '1'; }();
   const int tr = 16 * p.R;
   p.w_rowcopy = (force_rowcopy || (tr < TC_M ? TC_M % tr : tr % TC_M)) ? 1 : 0;
@@ -364,7 +366,7 @@ static void launch_gemm_tc(const b200_engine* e, TcParams p, cudaStream_t st) {
   {  // activation tiles: 64 elements along K x NT tokens, written in the 128-byte-swizzle layout; tokens beyond T read as zero
     const cuuint64_t gdim[2] = {(cuuint64_t)p.K, (cuuint64_t)p.T};
     const cuuint64_t gstr[1] = {(cuuint64_t)p.K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)TC_KC, (cuuint32_t)(NT > 256 ? NT / 2 : NT)};
+    const cuuint32_t box[2] = {(cuuint32_t)TC_KC, (cuuint32_t)p.NT};
     encode_map(&maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.x16, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_128B);
   }
   if (!p.w_rowcopy) {
@@ -383,9 +385,7 @@ static void launch_gemm_tc(const b200_engine* e, TcParams p, cudaStream_t st) {
       }
     }
   }
-  dim3 grid(p.ntiles_m, (p.T + NT - 1) / NT, p.ksplit);
-  gemm_tc_kernel<<<grid, TC_THREADS, tc_smem_bytes(NT, p.a_stages, p.b_stages, p.w_stages, p.w_stage_bytes, p.nslab), st>>>(p, maps);
-  CK(cudaGetLastError());
+  launch_pdl(e->use_pdl, gemm_tc_kernel, dim3(plan.grid), dim3(TC_THREADS), tc_smem_bytes(p.NT, p.b_stages, p.w_stages, p.w_stage_bytes), st, p, maps);
 }
 
 // B200_ATTN_CLUSTER=1 runs the engine's attention as one thread-block cluster per head
@@ -506,33 +506,13 @@ static int launch_linear(b200_engine* e, GemvParams p, int batch, cudaStream_t s
     return 1;
   }
   __half* x16 = static_cast<__half*>(x16_buf ? x16_buf : e->d_x16);
-  to_half_kernel<<<batch, TOH_THREADS, 0, st>>>(p.x, p.x_stride, p.norm_w, p.eps, p.K, x16);
-  CK(cudaGetLastError());
+  launch_pdl(e->use_pdl, to_half_kernel, dim3(batch), dim3(TOH_THREADS), 0, st, p.x, p.x_stride, p.norm_w, p.eps, p.K, x16);
   TcParams t{};
   for (int s = 0; s < p.nseg; ++s) t.seg[s] = p.seg[s];
   t.nseg = p.nseg; t.K = p.K; t.x16 = x16; t.T = batch; t.epi = p.epi; t.y = p.y; t.y_stride = p.y_stride; t.y2 = p.y2;
   t.y2_stride = p.y2_stride; t.resid = p.resid; t.rope = p.rope; t.positions = p.positions; t.head_dim = p.head_dim; t.max_pos = p.max_pos;
+  launch_gemm_tc(e, t, st);
   int n = 2;
-  // Few row tiles (O and down projections: 32 for a 4096-row matrix) leave most SMs idle: split K over
-  // up to 8 CTAs per tile, partial outputs summed in order by a small kernel (with the residual).
-  const int ctas = (int)((p.seg[0].rows + TC_M - 1) / TC_M) * ((batch + TC_MAX_N - 1) / TC_MAX_N);
-  const int nblk = p.K / 256;
-  int ks = 1;
-  if ((p.epi == EPI_RESID || (p.epi == EPI_STORE && !p.amax_val)) && p.nseg == 1 && batch <= 512 && e->d_tc_part) ks = std::max(1, std::min({8, e->num_sms / std::max(1, ctas), nblk / 4}));
-  if (ks > 1) {
-    t.ksplit = ks; t.kblocks = (nblk + ks - 1) / ks;
-    t.ksplit = (nblk + t.kblocks - 1) / t.kblocks;  // no empty split
-    t.epi = EPI_STORE; t.y = e->d_tc_part; t.y_stride = p.seg[0].rows;
-    launch_gemm_tc(e, t, st);
-    const size_t nel = (size_t)batch * p.seg[0].rows;
-    if (p.seg[0].rows % 4 || p.y_stride % 4) throw std::runtime_error("split-K matmul: rows must be a multiple of 4");
-    splitk_reduce_kernel<<<(unsigned)std::min<size_t>((nel / 4 + 255) / 256, 1184), 256, 0, st>>>(e->d_tc_part, t.ksplit, batch, p.seg[0].rows, p.resid, p.epi == EPI_RESID ? 1 : 0, p.y,
-                                                                                                   p.y_stride);
-    CK(cudaGetLastError());
-    ++n;
-  } else {
-    launch_gemm_tc(e, t, st);
-  }
   if (p.amax_val) {  // lm_head: the matvec kernel leaves argmax partials; here a small kernel scans the logits
     argmax_rows_kernel<<<batch, 256, 0, st>>>(p.y, p.y_stride, p.amax_row_offset, p.amax_val, p.amax_idx);
     CK(cudaGetLastError());

@@ -204,7 +204,7 @@ static void stage_release(b200_engine* e) {
   }
 }
 
-// Uploads one packed tensor and lays it out on the device as the stage images the matvec kernel
+// Uploads one packed tensor and lays it out on the device as the cells the matvec kernel
 // streams (Q6_K / Q8_0 are first regrouped into aligned 256-element units). half >= 0: the tensor
 // is the gate (0) or up (1) projection and shares its image with the other one, every 16-row
 // group holding eight gate rows and the same eight up rows.
@@ -253,7 +253,7 @@ static void upload_packed(b200_engine* e, DevTensor& t, int type, const void* ho
     CK(cudaGetLastError());
     usrc = units;
   }
-  stage_image_kernel<<<1184, 256, 0, stream>>>(usrc, dsrc, rows, g, half, t.base);
+  stage_image_kernel<<<1184, 256, 0, stream>>>(usrc, dsrc, rows, g, gemv_cell_bytes(type), half, t.base);
   CK(cudaGetLastError());
   // no synchronisation here: the scratch buffers are reused by the next tensor on the same stream, in order
 }
@@ -262,8 +262,7 @@ static GemvSeg seg_of(const DevTensor& t) {
   const GemvGeom g = gemv_geometry(t.type, (int)t.cols);
   GemvSeg s;
   s.img = t.base; s.type = t.type; s.rows = (int)t.img_rows; s.tiles = t.tiles;
-  s.RS = g.RS; s.RS_last = g.RS_last; s.d_off = g.d_off; s.d_off_last = g.d_off_last;
-  s.stage_bytes = g.stage_bytes; s.stage_bytes_last = g.stage_bytes_last; s.tile_bytes = g.tile_bytes;
+    s.stage_bytes = g.stage_bytes; s.stage_bytes_last = g.stage_bytes_last; s.tile_bytes = g.tile_bytes;
   return s;
 }
 
@@ -337,55 +336,36 @@ static void encode_map(CUtensorMap* tm, CUtensorMapDataType dt, int rank, const 
 
 static void launch_gemm_tc(const b200_engine* e, TcParams p, cudaStream_t st) {
   set_gemv_attrs();
-  const GemvGeom g0 = gemv_geometry(p.seg[0].type, p.K);
-  p.nblk = g0.nblk; p.nslab = g0.nslab; p.S = g0.S; p.S_last = g0.S_last; p.R = g0.R;
+  p.nblk = p.K / 256;
   const int tiles_n0 = (p.T + TC_MAX_N - 1) / TC_MAX_N;
   p.NT = ((p.T + tiles_n0 - 1) / tiles_n0 + 31) / 32 * 32;  // token tiles of equal width
   p.tiles_n = (p.T + p.NT - 1) / p.NT;
-  int tiles_m = 0, ub_max = 0;
+  int tiles_m = 0, cell = 0;
   for (int s = 0; s < p.nseg; ++s) {
     tiles_m += (p.seg[s].rows + TC_M - 1) / TC_M;
-    ub_max = std::max(ub_max, gemv_unit_bytes(p.seg[s].type));
+    cell = std::max(cell, gemv_cell_bytes(p.seg[s].type));
   }
   p.error_flag = e->d_error;
   p.ws = e->d_tc_part;
   p.tickets = e->d_tc_tickets;
   const TcPlan plan = tc_plan(tiles_m * p.tiles_n, p.nblk, p.NT, e->num_sms, p.ws != nullptr);
   p.rem = plan.rem; p.ge = plan.ge; p.full = plan.full;
-  // shared memory: 128 KB of activation stages for the widest token tiles (four steps ahead), eight stages for narrow ones; the
-  // rest for packed units, whose trip from HBM the kernel lives on when there are few tokens
-  p.w_stage_bytes = (TC_M * ub_max + 127) / 128 * 128;
-  p.b_stages = p.NT > 192 ? 4 : p.NT > 128 ? 5 : p.NT > 64 ? 6 : TC_B_STAGES;
+  // shared memory: up to 128 KB of activation stages (a copy covers as many steps as 32 KB hold), the rest for packed units,
+  // whose trip from HBM the kernel lives on when there are few tokens
+  p.w_stage_bytes = 8 * cell;
+  p.bk = p.NT <= 64 ? 4 : p.NT <= 128 ? 2 : 1;
+  p.b_stages = p.NT <= 64 ? 3 : 4;
   p.w_stages = TC_W_STAGES;
-  while (p.w_stages > 1 && tc_smem_bytes(p.NT, p.b_stages, p.w_stages, p.w_stage_bytes) > (size_t)TC_SMEM_MAX) --p.w_stages;
-  static const bool force_rowcopy = [] { const char* v = std::getenv("B200_TC_ROWCOPY"); return v && v[0] == '1'; }();
-  const int tr = 16 * p.R;
-  p.w_rowcopy = (force_rowcopy || (tr < TC_M ? TC_M % tr : tr % TC_M)) ? 1 : 0;
+  while (p.w_stages > 1 && tc_smem_bytes(p.NT, p.bk, p.b_stages, p.w_stages, p.w_stage_bytes) > (size_t)TC_SMEM_MAX) --p.w_stages;
   TcMaps maps;
   std::memset(&maps, 0, sizeof(maps));
-  {  // activation tiles: 64 elements along K x NT tokens, written in the 128-byte-swizzle layout; tokens beyond T read as zero
-    const cuuint64_t gdim[2] = {(cuuint64_t)p.K, (cuuint64_t)p.T};
-    const cuuint64_t gstr[1] = {(cuuint64_t)p.K * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)TC_KC, (cuuint32_t)p.NT};
-    encode_map(&maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.x16, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_128B);
+  {  // activation stages: bk steps of 64 elements x NT tokens, each step in the 128-byte-swizzle layout; tokens beyond T read as zero
+    const cuuint64_t gdim[3] = {(cuuint64_t)TC_KC, (cuuint64_t)p.T, (cuuint64_t)(p.K / TC_KC)};
+    const cuuint64_t gstr[2] = {(cuuint64_t)p.K * 2, (cuuint64_t)TC_KC * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)TC_KC, (cuuint32_t)p.NT, (cuuint32_t)p.bk};
+    encode_map(&maps.act, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, p.x16, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_128B);
   }
-  if (!p.w_rowcopy) {
-    // packed units: (32-bit words of a stage row, rows of an image tile, slabs, image tiles); box = one unit x 128 rows
-    for (int s = 0; s < p.nseg; ++s) {
-      const GemvSeg& sg = p.seg[s];
-      const cuuint32_t ub = (cuuint32_t)gemv_unit_bytes(sg.type);
-      const cuuint32_t box[4] = {ub / 4, (cuuint32_t)std::min(tr, TC_M), 1, (cuuint32_t)std::max(1, TC_M / tr)};
-      for (int last = 0; last < 2; ++last) {
-        if (!last && p.nslab == 1) continue;
-        const cuuint64_t rs = (cuuint64_t)(last ? sg.RS_last : sg.RS);
-        const cuuint64_t gdim[4] = {rs / 4, (cuuint64_t)tr, (cuuint64_t)(last ? 1 : p.nslab - 1), (cuuint64_t)sg.tiles};
-        const cuuint64_t gstr[3] = {rs, (cuuint64_t)(last ? sg.stage_bytes_last : sg.stage_bytes), (cuuint64_t)sg.tile_bytes};
-        const uint8_t* base = sg.img + (last ? (size_t)(p.nslab - 1) * sg.stage_bytes : 0);
-        encode_map(&maps.w[s][last], CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, base, gdim, gstr, box, CU_TENSOR_MAP_SWIZZLE_NONE);
-      }
-    }
-  }
-  launch_pdl(e->use_pdl, gemm_tc_kernel, dim3(plan.grid), dim3(TC_THREADS), tc_smem_bytes(p.NT, p.b_stages, p.w_stages, p.w_stage_bytes), st, p, maps);
+  launch_pdl(e->use_pdl, gemm_tc_kernel, dim3(plan.grid), dim3(TC_THREADS), tc_smem_bytes(p.NT, p.bk, p.b_stages, p.w_stages, p.w_stage_bytes), st, p, maps);
 }
 
 // B200_ATTN_CLUSTER=1 runs the engine's attention as one thread-block cluster per head

@@ -13,7 +13,7 @@ namespace b200 {
 struct DevTensor {
   int type = -1;
   int64_t rows = 0, cols = 0;  // logical shape
-  uint8_t* base = nullptr;     // packed types: stage images (see gemv.cuh); F32: the data
+  uint8_t* base = nullptr;     // packed types: cells (see gemv.cuh); F32: the data
   size_t bytes = 0;            // packed bytes as in the file (the algorithmic byte count)
   int64_t img_rows = 0;        // rows the image holds data for (2 x rows for the gate+up image)
   int tiles = 0;               // image tiles of 16*R rows

@@ -4,17 +4,18 @@
 // (model.cpp:2141-2249). "Swap-AB": the weight rows are the M side of the MMA (128 per tile), the tokens
 // the N side (32..256 per tile).
 //
-// One persistent CTA (608 threads) per SM walks K in steps of 64 elements, four to a packed block:
-//   * a weight-producer lane brings the packed units of the tile's 128 rows, one 256-element block
-//     per tensor copy (cp.async.bulk.tensor.4d over the stage images), into a ring;
+// One persistent CTA (608 threads) per SM walks K block by block, four steps of 64 elements to a block:
+//   * a weight-producer warp brings the packed units of the tile's 128 rows, one 256-element block at a time as eight
+//     contiguous cells (cp.async.bulk), into a ring;
 //   * sixteen warps dequantise into TENSOR MEMORY, which is where the MMA takes its A operand from:
-//     thread = (weight row = TMEM lane, one 64-element step of the block), so that the four warps of a
-//     step are the only writers of its stage (32 columns of packed fp16 pairs, eight stages) and one
-//     wait, one fence and one arrival cover 64 elements of a thread;
+//     thread = (weight row = TMEM lane, one 64-element step of the block), 32 columns of packed fp16 pairs a
+//     step, two blocks; one wait, one fence and one arrival cover 64 elements of a thread;
 //   * an activation-producer lane moves the matching slices of the fp16 activations with TMA
-//     (cp.async.bulk.tensor.2d, 128-byte swizzle, tokens beyond T read as zero);
-//   * one lane of the MMA warp issues four tcgen05.mma (M=128, N=NT, K=16, kind::f16) per step into an
-//     fp32 accumulator in tensor memory (two of them when NT <= 128);
+//     (cp.async.bulk.tensor.3d, 128-byte swizzle, tokens beyond T read as zero), one to four steps a copy;
+//   * the MMA warp issues sixteen tcgen05.mma (M=128, N=NT, K=16, kind::f16) per block into an
+//     fp32 accumulator in tensor memory (two of them when NT <= 128). Its instruction stream is serial: as a
+//     branch for one lane, with two waits and a commit a step, it took 860 cycles a step, whatever NT, and everyone
+//     waited for it; so the warp runs it together, with few waits, and one lane is elected for the MMAs alone;
 //   * after a unit's last step the sixteen warps read their TMEM lanes back (tcgen05.ld 32x32b: thread =
 //     weight row, registers = tokens) and run the matvec kernel's epilogues.
 // The roles meet on mbarriers only. Every wait is bounded; on a give-up the kernel sets the error word,
@@ -50,7 +51,7 @@ struct TcParams {
   GemvSeg seg[3];
   int nseg;
   int K;
-  int nblk, nslab, S, S_last, R;  // GemvGeom of K (where a unit sits inside the stage images)
+  int nblk;                       // 256-element blocks along K
   const __half* x16;              // [T][K] activations (already normalised when the layer asks for it)
   int T;                          // tokens
   int NT;                         // tokens per tile: a multiple of 32, <= 256
@@ -65,9 +66,8 @@ struct TcParams {
   int head_dim, max_pos;
   int tiles_n;                    // token tiles; tile = row tile * tiles_n + token tile
   int rem, ge, full;              // tiles 0 .. rem-1 are cut into ge ranges along K, the others run whole, `full` per CTA
-  int b_stages;                   // activation stages
-  int w_stages, w_stage_bytes;    // packed-weight ring: stages of 128 rows x unit bytes
-  int w_rowcopy;                  // 1: the producer copies row by row (geometries a tensor map cannot describe)
+  int bk, b_stages;               // steps of an activation stage (1, 2 or 4), stages
+  int w_stages, w_stage_bytes;    // packed-weight ring: stages of eight cells
   float* ws;                      // partial sums of cut tiles, [2 * ge][NT][128]
   int* tickets;                   // one per cut tile, zero between launches
   int* error_flag;
@@ -92,14 +92,29 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t desc_a, uin
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
-// the same with A in tensor memory: lane = row, each 32-bit column two consecutive elements along K
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// the same with A in tensor memory: lane = row, each 32-bit column two consecutive elements along K. The whole warp calls it,
+// the leader issues it: control flow and addresses stay uniform over the warp (uniform registers, which the instruction wants)
+__device__ __forceinline__ void tc_mma_f16_ts(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(uint32_t leader, void* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(smem_u32(bar)), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t warp_leader() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(r));
+  return r;
 }
 // thread = lane, 16 consecutive columns from registers
 __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -176,33 +191,36 @@ __device__ __forceinline__ void tc_affine4(uint32_t bytes, uint64_t D, uint64_t 
 __device__ __forceinline__ uint32_t u4_word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
 // The packed bytes one thread needs for its 64 elements [64 c, 64 c + 64) of a block, copied from the ring so that
-// the stage can be refilled while they are converted.
+// the stage can be refilled while they are converted. cell, r: the row's cell and its row in it.
 //   Q4_K: r[0] = d, dmin, 12 scale bytes; r[1..2] = 32 nibble pairs (low nibbles = elements 0..31, high = 32..63)
 //   Q6_K: r[0..3] = ql bytes, r[4..5] = qh bytes of the 128-element half; aux = four sub-block scales; d = block scale
 //   Q8_0: r[0..3] = 64 quants; aux = two fp16 scales
-// Bank conflicts: rows lie 144, 208 or 272 bytes apart, so eight lanes' 16-byte loads fall in distinct banks.
 struct TcRaw {
   uint4 r[6];
   uint32_t aux;
+  uint16_t d;
 };
 
 template <int TYPE>
-__device__ __forceinline__ void tc_fetch(const uint8_t* unit, int c, TcRaw& t) {
+__device__ __forceinline__ void tc_fetch(const uint8_t* cell, int r, int c, TcRaw& t) {
+  const uint8_t* even = cell + 16 * r;                  // chunk 0 of the row; chunk n lies 256 n further,
+  const uint8_t* odd = cell + 16 * (r ^ 4);             // odd chunks in the row's swapped place
   if (TYPE == T_Q4_K) {
-    t.r[0] = *reinterpret_cast<const uint4*>(unit);
-    t.r[1] = *reinterpret_cast<const uint4*>(unit + 16 + 32 * c);
-    t.r[2] = *reinterpret_cast<const uint4*>(unit + 32 + 32 * c);
+    t.r[0] = *reinterpret_cast<const uint4*>(even);
+    t.r[1] = *reinterpret_cast<const uint4*>(odd + 256 * (1 + 2 * c));
+    t.r[2] = *reinterpret_cast<const uint4*>(even + 256 * (2 + 2 * c));
   } else if (TYPE == T_Q6_K) {
     const int hh = c >> 1;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t.r[i] = *reinterpret_cast<const uint4*>(unit + 64 * hh + 16 * i);
+    for (int i = 0; i < 4; ++i) t.r[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + 256 * (4 * hh + i));
 #pragma unroll
-    for (int i = 0; i < 2; ++i) t.r[4 + i] = *reinterpret_cast<const uint4*>(unit + 128 + 32 * hh + 16 * i);
-    t.aux = *reinterpret_cast<const uint32_t*>(unit + 192 + 4 * c);
+    for (int i = 0; i < 2; ++i) t.r[4 + i] = *reinterpret_cast<const uint4*>((i ? odd : even) + 256 * (8 + 2 * hh + i));
+    t.aux = *reinterpret_cast<const uint32_t*>(even + 256 * 12 + 4 * c);
+    t.d = *reinterpret_cast<const uint16_t*>(cell + 16 * 208 + 2 * r);
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t.r[i] = *reinterpret_cast<const uint4*>(unit + 64 * c + 16 * i);
-    t.aux = *reinterpret_cast<const uint32_t*>(unit + 256 + 4 * c);
+    for (int i = 0; i < 4; ++i) t.r[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + 256 * (4 * c + i));
+    t.aux = *reinterpret_cast<const uint32_t*>(even + 256 * 16 + 4 * c);
   }
 }
 
@@ -212,7 +230,7 @@ __device__ __forceinline__ void tc_fetch(const uint8_t* unit, int c, TcRaw& t) {
 // dequantize_q6_k / dequantize_q8_0_block (quantization.cpp:171-266, 1047-1052). FP32 pairs (fma.rn.f32x2) halve the
 // multiply-adds; what is left per element is one byte permute and half a conversion.
 template <int TYPE>
-__device__ __forceinline__ void tc_dequant32(const TcRaw& t, uint16_t dbits, int c, int hf, uint32_t (&w)[16]) {
+__device__ __forceinline__ void tc_dequant32(const TcRaw& t, int c, int hf, uint32_t (&w)[16]) {
   if (TYPE == T_Q4_K) {
     const uint4 h = t.r[0];
     const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(&h.x));
@@ -234,7 +252,7 @@ __device__ __forceinline__ void tc_dequant32(const TcRaw& t, uint16_t dbits, int
   } else if (TYPE == T_Q6_K) {
     // 32-element group 2 (c & 1) + hf of the 128-element half: low nibbles of ql (high ones for the upper two groups),
     // two bits of qh brought to bits 4-5 by one rotation, one bitwise select, one more clears bits 6-7 and sets bit 7
-    const float d = half_bits_to_float(dbits);
+    const float d = half_bits_to_float(t.d);
     const int lsh = 4 * (c & 1), hrot = (4 - 2 * hf - 4 * (c & 1)) & 31;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
@@ -264,22 +282,18 @@ __device__ __forceinline__ void tc_dequant32(const TcRaw& t, uint16_t dbits, int
 }
 
 constexpr int TC_B_STAGES = 8;   // at most: activation tiles in flight (TMA)
-constexpr int TC_A_STAGES = 8;   // weight stages in tensor memory, 32 columns each: two blocks
-constexpr int TC_W_STAGES = 6;   // at most: packed-weight stages in flight (TMA)
-constexpr uint32_t TC_A_COL = 256;  // first tensor-memory column of the weight stages (the accumulators lie below)
+constexpr int TC_W_STAGES = 8;   // at most: packed-weight stages in flight (TMA)
+constexpr uint32_t TC_A_COL = 256;  // first tensor-memory column of the two weight blocks, 128 columns each (the accumulators lie below)
 
-// Tensor maps of one launch: the fp16 activations and, per segment, the packed units of its stage
-// images seen as a 4-D array (bytes of a stage row / rows of an image tile / slabs / image tiles) -
-// one map for the full slabs and one for the last slab of every tile, whose rows are shorter.
 struct alignas(64) TcMaps {
-  CUtensorMap act;
-  CUtensorMap w[3][2];
+  CUtensorMap act;  // the fp16 activations
 };
 
 struct TcShared {
-  unsigned long long a_full[TC_A_STAGES];    // the four warps of a step have stored its weights
+  unsigned long long a_full[2];              // the sixteen warps have stored a block's weights
+  unsigned long long a_empty[2];             // the MMAs that read them have completed
   unsigned long long b_full[TC_B_STAGES];    // the activation tile has landed (TMA transaction bytes)
-  unsigned long long mma_done[TC_A_STAGES];  // the MMAs of the step in weight stage i (and its activation stage) have completed
+  unsigned long long b_empty[TC_B_STAGES];   // the MMAs that read it have completed
   unsigned long long acc_full[2];            // all MMAs of a unit have completed
   unsigned long long acc_empty[2];           // the sixteen warps have read the accumulator
   unsigned long long w_full[TC_W_STAGES];    // the packed units of a block have landed
@@ -310,22 +324,22 @@ __device__ __forceinline__ bool tc_wait(const TcParams& p, TcShared* sh, void* b
 }
 __device__ __forceinline__ void tc_workers_sync() { asm volatile("bar.sync 14, %0;" ::"n"(TC_WORKERS) : "memory"); }
 
-// 2-D tiled TMA load of one activation tile (64 elements along K x NT tokens, 128-byte swizzle)
+// 2-D tiled TMA load (64 elements along K x rows, 128-byte swizzle)
 __device__ __forceinline__ void tc_tma_load_2d(void* dst, const void* tmap, int c0, int c1, void* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
                "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
                : "memory");
 }
-// 4-D tiled TMA load of the packed units of 128 rows of one block (no swizzle: rows land back to back)
-__device__ __forceinline__ void tc_tma_load_4d(void* dst, const void* tmap, int c0, int c1, int c2, int c3, void* bar) {
-  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(dst)),
-               "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+// 3-D tiled TMA load of an activation stage: steps x NT tokens x 64 elements, each step a tile in the 128-byte swizzle
+__device__ __forceinline__ void tc_tma_load_3d(void* dst, const void* tmap, int c0, int c1, int c2, void* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+               "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
 
-// Dynamic shared memory (1024-byte aligned): the activation stages of NT x 128 bytes, then the packed-weight ring.
-__host__ __device__ __forceinline__ size_t tc_smem_bytes(int NT, int b_stages, int w_stages, int w_stage_bytes) {
-  return 1024 + b_stages * (size_t)NT * 128 + (size_t)w_stages * w_stage_bytes;
+// Dynamic shared memory (1024-byte aligned): the activation stages of bk x NT x 128 bytes, then the packed-weight ring.
+__host__ __device__ __forceinline__ size_t tc_smem_bytes(int NT, int bk, int b_stages, int w_stages, int w_stage_bytes) {
+  return 1024 + (size_t)b_stages * bk * NT * 128 + (size_t)w_stages * w_stage_bytes;
 }
 constexpr int TC_SMEM_MAX = 226 * 1024;  // dynamic part; the barriers live in static shared memory
 
@@ -449,46 +463,30 @@ __device__ __forceinline__ void tc_finish8(const TcParams& p, const TcWork& w, i
 // One unit's blocks by a dequantising warp; blk: blocks of this CTA before it (ring position).
 template <int TYPE>
 __device__ __forceinline__ void tc_dequant_unit(const TcParams& p, TcShared& sh, const uint8_t* Wbase, uint32_t tmem, const TcWork& w, int blk) {
-  constexpr int ub = TYPE == T_Q4_K ? 144 : TYPE == T_Q6_K ? 208 : 272;
+  constexpr int cell = TYPE == T_Q4_K ? 16 * 144 : TYPE == T_Q6_K ? 16 * 208 + 32 : 16 * 272;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int my_row = threadIdx.x & (TC_M - 1), c = warp >> 2;
   const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
-  const GemvSeg& sg = p.seg[w.seg];
-  // Q6_K: the fp16 scales of a row's blocks follow its units in the stage row; one block ahead, from global memory (a
-  // row's scales of a slab share a sector)
-  const int irow = min(w.row0 + my_row, sg.rows - 1), tr = 16 * p.R;
-  const uint8_t* const dtile = sg.img + (size_t)(irow / tr) * sg.tile_bytes;
-  const int rr = irow % tr;
-  auto dload = [&](int gb) -> uint16_t {
-    if (TYPE != T_Q6_K) return 0;
-    const int slab = gb / p.S, bb = gb - slab * p.S;
-    const bool last = slab == p.nslab - 1;
-    return __ldg(reinterpret_cast<const uint16_t*>(dtile + (size_t)slab * sg.stage_bytes + (size_t)rr * (last ? sg.RS_last : sg.RS) +
-                                                   (last ? sg.d_off_last : sg.d_off) + 2 * bb));
-  };
-  uint16_t dnext = dload(w.b0);
   int stage = blk % p.w_stages;
   uint32_t wpar = (uint32_t)((blk / p.w_stages) & 1);
 #pragma unroll 1
   for (int i = 0; i < w.nb; ++i, ++blk) {
-    const uint16_t dcur = dnext;
-    if (TYPE == T_Q6_K && i + 1 < w.nb) dnext = dload(w.b0 + i + 1);
     tc_wait(p, &sh, &sh.w_full[stage], wpar);
     TcRaw raw;
-    tc_fetch<TYPE>(Wbase + (size_t)stage * p.w_stage_bytes + (size_t)my_row * ub, c, raw);
+    tc_fetch<TYPE>(Wbase + (size_t)stage * p.w_stage_bytes + (size_t)(my_row >> 4) * cell, my_row & 15, c, raw);
     uint32_t v[16];
-    tc_dequant32<TYPE>(raw, dcur, c, 0, v);
+    tc_dequant32<TYPE>(raw, c, 0, v);
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh.w_empty[stage]);  // the stage may be refilled
     if (++stage == p.w_stages) { stage = 0; wpar ^= 1u; }
-    // the MMAs that read this weight stage two blocks ago must be done before it is overwritten
-    const int sa = 4 * (blk & 1) + c;
-    if (blk >= 2) tc_wait(p, &sh, &sh.mma_done[sa], (uint32_t)(((blk >> 1) - 1) & 1));
+    // the MMAs that read this half of the weight columns two blocks ago must be done before it is overwritten
+    const int sa = blk & 1;
+    if (blk >= 2) tc_wait(p, &sh, &sh.a_empty[sa], (uint32_t)(((blk >> 1) - 1) & 1));
     tc_fence_after();
-    const uint32_t dst = tmem + TC_A_COL + 32u * (uint32_t)sa + lanes;
+    const uint32_t dst = tmem + TC_A_COL + 32u * (uint32_t)(4 * sa + c) + lanes;
     __syncwarp();
     tc_st16(dst, v);
-    tc_dequant32<TYPE>(raw, dcur, c, 1, v);
+    tc_dequant32<TYPE>(raw, c, 1, v);
     tc_st16(dst + 16, v);
     tc_wait_st();
     tc_fence_before();
@@ -504,13 +502,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
   extern __shared__ uint8_t tc_smem_raw[];
   __shared__ TcShared sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  uint8_t* const Bbase = reinterpret_cast<uint8_t*>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);  // [b_stages][NT rows][128 B]
-  const uint32_t b_stage_bytes = (uint32_t)p.NT * 128;
+  uint8_t* const Bbase = reinterpret_cast<uint8_t*>(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);  // [b_stages][bk][NT rows][128 B]
+  const uint32_t b_stage_bytes = (uint32_t)(p.bk * p.NT) * 128;
   uint8_t* const Wbase = Bbase + (size_t)p.b_stages * b_stage_bytes;  // [w_stages][128 rows][unit bytes]
   const int nbuf = p.NT <= (int)TC_A_COL / 2 ? 2 : 1;                 // accumulators, 128 columns apart
   if (tid == 0) {
-    for (int i = 0; i < TC_A_STAGES; ++i) { mbar_init(&sh.a_full[i], 4); mbar_init(&sh.mma_done[i], 1); }
-    for (int i = 0; i < TC_B_STAGES; ++i) mbar_init(&sh.b_full[i], 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&sh.a_full[i], TC_WORKERS / 32); mbar_init(&sh.a_empty[i], 1); }
+    for (int i = 0; i < TC_B_STAGES; ++i) { mbar_init(&sh.b_full[i], 1); mbar_init(&sh.b_empty[i], 1); }
     for (int i = 0; i < TC_W_STAGES; ++i) { mbar_init(&sh.w_full[i], 1); mbar_init(&sh.w_empty[i], TC_WORKERS / 32); }
     for (int i = 0; i < 2; ++i) { mbar_init(&sh.acc_full[i], 1); mbar_init(&sh.acc_empty[i], TC_WORKERS / 32); }
     sh.abort_flag = 0;
@@ -526,89 +524,92 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
   TcWork w;
 
   if (warp == TC_WORKERS / 32) {
-    // ---- MMA warp: one lane waits for a weight stage and an activation stage and issues the step's four MMAs ----
-    if (lane == 0) {
-      const uint32_t idesc = tc_idesc(p.NT);
-      const uint64_t bdesc0 = tc_smem_desc(smem_u32(Bbase)), b_step = (uint64_t)(b_stage_bytes >> 4);
-      int sa = 0, sb = 0;
-      uint32_t pa = 0, pb = 0;
-      uint64_t bdesc = bdesc0;
-      bool ok = true;
-      for (int u = 0; ok && tc_work(p, blockIdx.x, u, w); ++u) {
-        const int buf = nbuf == 2 ? (u & 1) : 0, use = nbuf == 2 ? (u >> 1) : u;
-        if (use > 0 && !(ok = tc_wait(p, &sh, &sh.acc_empty[buf], (uint32_t)((use - 1) & 1)))) break;
-        tc_fence_after();
-        const uint32_t d = tmem + 128u * (uint32_t)buf;
+    // ---- MMA warp ----
+    const uint32_t leader = warp_leader();
+    const uint32_t idesc = tc_idesc(p.NT);
+    const uint64_t bdesc0 = tc_smem_desc(smem_u32(Bbase)), b_step = (uint64_t)((p.NT * 128) >> 4);
+    int sb = 0, blk = 0;
+    uint32_t pb = 0;
+    uint64_t bdesc = bdesc0;
+    bool ok = true;
+    auto wait = [&](void* bar, uint32_t parity) { return __all_sync(0xffffffffu, tc_wait(p, &sh, bar, parity)) != 0; };
+    for (int u = 0; ok && tc_work(p, blockIdx.x, u, w); ++u) {
+      const int buf = nbuf == 2 ? (u & 1) : 0, use = nbuf == 2 ? (u >> 1) : u;
+      if (use > 0 && !(ok = wait(&sh.acc_empty[buf], (uint32_t)((use - 1) & 1)))) break;
+      const uint32_t d = tmem + 128u * (uint32_t)buf;
+      uint32_t accumulate = 0;
 #pragma unroll 1
-        for (int s = 0; s < 4 * w.nb; ++s) {
-          if (!(ok = tc_wait(p, &sh, &sh.b_full[sb], pb) && tc_wait(p, &sh, &sh.a_full[sa], pa))) break;
+      for (int i = 0; i < w.nb; ++i, ++blk) {
+        const int sa = blk & 1;
+        if (!(ok = wait(&sh.a_full[sa], (uint32_t)((blk >> 1) & 1)))) break;
+        uint32_t a = tmem + TC_A_COL + 128u * (uint32_t)sa;
+#pragma unroll 1
+        for (int k = 0; k < 4; k += p.bk) {
+          if (!(ok = wait(&sh.b_full[sb], pb))) break;
           tc_fence_after();
-          const uint32_t a = tmem + TC_A_COL + 32u * (uint32_t)sa;
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4)  // 16 elements along K = 8 columns of A, 32 bytes = 2 descriptor units of B
-            tc_mma_f16_ts(d, a + 8 * k4, bdesc + 2 * k4, idesc, (s | k4) ? 1u : 0u);
-          tc_commit(&sh.mma_done[sa]);
-          bdesc += b_step;
-          if (++sa == TC_A_STAGES) { sa = 0; pa ^= 1u; }
+#pragma unroll 1
+          for (int j = 0; j < p.bk; ++j) {
+            tc_mma_f16_ts(leader, d, a, bdesc, idesc, accumulate);  // 16 elements along K = 8 columns of A, 32 bytes = 2 descriptor units of B
+            tc_mma_f16_ts(leader, d, a + 8, bdesc + 2, idesc, 1u);
+            tc_mma_f16_ts(leader, d, a + 16, bdesc + 4, idesc, 1u);
+            tc_mma_f16_ts(leader, d, a + 24, bdesc + 6, idesc, 1u);
+            accumulate = 1u;
+            a += 32;
+            bdesc += b_step;
+          }
+          tc_commit_if(leader, &sh.b_empty[sb]);
           if (++sb == p.b_stages) { sb = 0; pb ^= 1u; bdesc = bdesc0; }
         }
-        if (ok) tc_commit(&sh.acc_full[buf]);
+        if (!ok) break;
+        tc_commit_if(leader, &sh.a_empty[sa]);
       }
+      if (ok) tc_commit_if(leader, &sh.acc_full[buf]);
     }
     __syncwarp();
   } else if (warp == TC_WORKERS / 32 + 2) {
-    // ---- activation producer: tile of step s into stage s % nb as soon as the MMAs of step s - nb have read it ----
+    // ---- activation producer ----
     if (lane == 0) {
       pdl_wait();
-      const int nb = p.b_stages;
-      int s = 0;
+      int sb = 0, n = 0;
+      uint32_t pb = 1;  // a fresh ring's stages count as empty
       bool ok = true;
       for (int u = 0; ok && tc_work(p, blockIdx.x, u, w); ++u) {
 #pragma unroll 1
-        for (int k = 0; k < 4 * w.nb; ++k, ++s) {
-          if (s >= nb && !(ok = tc_wait(p, &sh, &sh.mma_done[(s - nb) % TC_A_STAGES], (uint32_t)(((s - nb) / TC_A_STAGES) & 1)))) break;
-          void* bar = &sh.b_full[s % nb];
-          mbar_expect_tx(bar, b_stage_bytes);
-          tc_tma_load_2d(Bbase + (size_t)(s % nb) * b_stage_bytes, &maps.act, (4 * w.b0 + k) * TC_KC, w.t0, bar);
-          *(volatile int*)&sh.b_issued = s + 1;
+        for (int k = 4 * w.b0; k < 4 * (w.b0 + w.nb); k += p.bk) {
+          if (n >= p.b_stages && !(ok = tc_wait(p, &sh, &sh.b_empty[sb], pb))) break;
+          mbar_expect_tx(&sh.b_full[sb], b_stage_bytes);
+          tc_tma_load_3d(Bbase + (size_t)sb * b_stage_bytes, &maps.act, 0, w.t0, k, &sh.b_full[sb]);
+          *(volatile int*)&sh.b_issued = ++n;
+          if (++sb == p.b_stages) { sb = 0; pb ^= 1u; }
         }
       }
     }
     __syncwarp();
   } else if (warp == TC_WORKERS / 32 + 1) {
-    // ---- weight producer: one tensor copy per 256-element block brings the packed units of the tile's 128 rows into the
-    //      ring (rows beyond the images read as zero) ----
-    const int tr = 16 * p.R, nw = p.w_stages;
+    // ---- weight producer: eight lanes copy the block's eight cells (row groups past the image repeat its last one; the
+    //      results of such rows are dropped) ----
+    const int nw = p.w_stages;
     int blk = 0;
     bool ok = true;
     for (int u = 0; ok && tc_work(p, blockIdx.x, u, w); ++u) {
       const GemvSeg& sg = p.seg[w.seg];
-      const int ub = gemv_unit_bytes(sg.type);
+      const uint32_t cell = (uint32_t)gemv_cell_bytes(sg.type);
+      const int group = min((w.row0 >> 4) + (lane & 7), (sg.rows - 1) >> 4);
+      const uint8_t* src = sg.img + ((size_t)group * p.nblk + w.b0) * cell;
 #pragma unroll 1
-      for (int i = 0; i < w.nb; ++i, ++blk) {
-        const int gb = w.b0 + i, slab = gb / p.S, bb = gb - slab * p.S;
-        const bool last = slab == p.nslab - 1;
+      for (int i = 0; i < w.nb; ++i, ++blk, src += cell) {
         const int stage = blk % nw;
         void* bar = &sh.w_full[stage];
-        uint8_t* dst = Wbase + (size_t)stage * p.w_stage_bytes;
         if (lane == 0) {
           ok = blk < nw || tc_wait(p, &sh, &sh.w_empty[stage], (uint32_t)((blk / nw - 1) & 1));
           if (ok) {
-            mbar_expect_tx(bar, (uint32_t)(TC_M * ub));
-            if (!p.w_rowcopy) tc_tma_load_4d(dst, &maps.w[w.seg][last ? 1 : 0], bb * ub / 4, w.row0 % tr, last ? 0 : slab, w.row0 / tr, bar);
+            mbar_expect_tx(bar, 8 * cell);
             *(volatile int*)&sh.w_issued = blk + 1;
           }
         }
         ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
         if (!ok) break;
-        if (p.w_rowcopy) {
-          for (int r = lane; r < TC_M; r += 32) {
-            const int irow = min(w.row0 + r, sg.rows - 1);  // rows past the segment repeat the last one; their results are dropped
-            const int tile = irow / tr, rr = irow - tile * tr;
-            const uint8_t* rowp = sg.img + (size_t)tile * sg.tile_bytes + (size_t)slab * sg.stage_bytes + (size_t)rr * (last ? sg.RS_last : sg.RS);
-            bulk_g2s(dst + (size_t)r * ub, rowp + (size_t)bb * ub, (uint32_t)ub, bar);
-          }
-        }
+        if (lane < 8) bulk_g2s(Wbase + (size_t)stage * p.w_stage_bytes + (size_t)lane * cell, src, cell, bar);
       }
     }
     __syncwarp();

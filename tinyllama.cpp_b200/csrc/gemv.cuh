@@ -13,10 +13,10 @@
 // The Q4_K minimum term and the Q6_K "-32" offset use per-sub-block sums of the activations, also
 // kept as digit bytes, and are evaluated with dp4a.
 //
-// Data movement. Weights live in HBM as "stage images": the matrix is cut into tiles of 16*R
-// rows and slabs of S <= 16 blocks along K, and each (tile, slab) is stored as one contiguous
-// run laid out exactly as it will sit in shared memory (rows padded to a stride = 32 mod 128 so
-// the fragment loads are free of bank conflicts). One persistent CTA per SM walks its tiles:
+// Data movement. Weights live in HBM as cells: one 256-element block of 16 consecutive rows, laid out as it will sit
+// in shared memory so that the fragment loads are free of bank conflicts; the cells of a row group follow one
+// another along K. The matrix is cut into tiles of 16*R rows and slabs of S <= 16 blocks along K, and every (tile,
+// slab) is one contiguous run of cells. One persistent CTA per SM walks its tiles:
 // 16 consumer warps and one producer warp. One lane of the producer requests every stage with ONE
 // bulk asynchronous copy (cp.async.bulk, completion counted on an mbarrier) into a ring of
 // shared-memory slots as soon as the slot is empty (a second mbarrier per slot counts the consumer
@@ -29,8 +29,7 @@
 // The kernel supports programmatic dependent launch: the producer never depends on the previous
 // kernel and starts at once; only the consumers wait for that kernel's results.
 //
-// HBM traffic per launch = the packed bytes of the rows (each read exactly once, plus the row
-// padding: 1.4 % for a 4096-wide Q4_K matrix) plus the activation vector.
+// HBM traffic per launch = the packed bytes of the rows (each read exactly once) plus the activation vector.
 #pragma once
 #include "common.cuh"
 #include "dequant.cuh"
@@ -48,11 +47,18 @@ constexpr int GEMV_SMEM_BUDGET = 208 * 1024;          // dynamic shared memory (
 
 // One "unit" per 256 elements of a row:
 //   Q4_K  unit = the 144-byte block exactly as in the file
-//   Q6_K  unit = 208 bytes: ql[128] | qh[64] | scales[16] of the block; the fp16 d of the S blocks
-//         of a stage row follow the row's units (a 210-byte block cannot sit on a 16-byte boundary)
+//   Q6_K  unit = 208 bytes: ql[128] | qh[64] | scales[16] of the block (a 210-byte block cannot sit on a 16-byte boundary)
 //   Q8_0  unit = 272 bytes: the 8 x 32 quants of eight consecutive blocks, then their 8 fp16 d
 // The byte count is that of the file in every case; nothing is expanded.
+//
+// A cell holds the units of 16 rows in 16-byte chunks: chunk c of row r lies at (16 c + (r ^ 4 (c & 1))) * 16. The matvec
+// kernel's eight-byte fragment loads (four rows x two neighbouring chunks per half warp) and the batched matmul's
+// 16-byte loads (eight rows, one chunk) then fall in distinct banks. Q6_K: the rows' fp16 d follow, 32 bytes.
+// (With rows end to end per slab the batched matmul fetched a block of 128 rows as 128 pieces of 144 bytes, at about 29
+// cycles a piece, four times what HBM takes; eight cells of 2304 contiguous bytes arrive at the rate of HBM.)
 __host__ __device__ __forceinline__ int gemv_unit_bytes(int type) { return type == T_Q4_K ? 144 : type == T_Q6_K ? 208 : 272; }
+__host__ __device__ __forceinline__ int gemv_cell_bytes(int type) { return 16 * gemv_unit_bytes(type) + (type == T_Q6_K ? 32 : 0); }
+__host__ __device__ __forceinline__ uint32_t gemv_chunk(int r, int c) { return (uint32_t)(16 * c + (r ^ (4 * (c & 1)))) * 16; }
 
 // How a [rows][K] matrix of one block type is cut into ring stages. nblk, nslab, S, S_last and R
 // depend on K only, so segments of different types in one launch share them.
@@ -62,12 +68,8 @@ struct GemvGeom {
   int S, S_last; // blocks per row in a full stage / in the last stage of a tile
   int R;         // 16-row groups per tile (> 1 only for short rows, so that all 16 warps have a task)
   int ub;        // unit bytes
-  int RS, RS_last;        // bytes between rows of a stage (= 32 mod 128)
-  int d_off, d_off_last;  // Q6_K: offset of the row's fp16 block scales within a stage row
   uint32_t stage_bytes, stage_bytes_last, tile_bytes;
 };
-
-__host__ __device__ __forceinline__ int gemv_pad_row(int bytes) { return (bytes + 95) / 128 * 128 + 32; }
 
 __host__ __device__ inline GemvGeom gemv_geometry(int type, int K) {
   GemvGeom g;
@@ -77,14 +79,10 @@ __host__ __device__ inline GemvGeom gemv_geometry(int type, int K) {
   g.S = (g.nblk + g.nslab - 1) / g.nslab;
   g.S_last = g.nblk - (g.nslab - 1) * g.S;
   g.R = g.nslab == 1 ? (GEMV_WARPS / g.nblk > 0 ? GEMV_WARPS / g.nblk : 1) : 1;
-  const int dfull = type == T_Q6_K ? (2 * g.S + 15) / 16 * 16 : 0, dlast = type == T_Q6_K ? (2 * g.S_last + 15) / 16 * 16 : 0;
-  g.d_off = g.S * g.ub;
-  g.d_off_last = g.S_last * g.ub;
-  g.RS = gemv_pad_row(g.S * g.ub + dfull);
-  g.RS_last = gemv_pad_row(g.S_last * g.ub + dlast);
-  g.stage_bytes = (uint32_t)(g.R * 16 * g.RS);
-  g.stage_bytes_last = (uint32_t)(g.R * 16 * g.RS_last);
-  g.tile_bytes = (uint32_t)(g.nslab - 1) * g.stage_bytes + g.stage_bytes_last;
+  const uint32_t cell = (uint32_t)gemv_cell_bytes(type);
+  g.stage_bytes = (uint32_t)(g.R * g.S) * cell;
+  g.stage_bytes_last = (uint32_t)(g.R * g.S_last) * cell;
+  g.tile_bytes = (uint32_t)(g.R * g.nblk) * cell;
   return g;
 }
 
@@ -95,9 +93,9 @@ __host__ __device__ __forceinline__ int64_t gemv_image_row(int64_t r, int half) 
 }
 
 // Scatters contiguous units [rows][nblk][ub] (and, for Q6_K, their fp16 scales [rows][nblk]) into
-// the stage images. The image must have been zeroed (padding, rows beyond the matrix).
+// the cells. The image must have been zeroed (rows beyond the matrix).
 __global__ void stage_image_kernel(const uint8_t* __restrict__ units, const uint16_t* __restrict__ dsrc, int64_t rows, GemvGeom g,
-                                   int half, uint8_t* __restrict__ img) {
+                                   int cell_bytes, int half, uint8_t* __restrict__ img) {
   const int cpu = g.ub / 16;
   const int64_t total = rows * g.nblk * cpu;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -107,12 +105,7 @@ __global__ void stage_image_kernel(const uint8_t* __restrict__ units, const uint
     const int64_t r = u / g.nblk;
     const int b = (int)(u - r * g.nblk);
     const int64_t dr = gemv_image_row(r, half);
-    const int64_t tile = dr / (16 * g.R);
-    const int rr = (int)(dr - tile * 16 * g.R);
-    const int slab = b / g.S, bb = b - slab * g.S;
-    const bool last = slab == g.nslab - 1;
-    uint8_t* dst = img + (size_t)tile * g.tile_bytes + (size_t)slab * g.stage_bytes + (size_t)rr * (last ? g.RS_last : g.RS) +
-                   (size_t)bb * g.ub + (size_t)c * 16;
+    uint8_t* dst = img + (size_t)((dr >> 4) * g.nblk + b) * cell_bytes + gemv_chunk((int)(dr & 15), c);
     *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(units + (size_t)u * g.ub + (size_t)c * 16);
   }
   if (dsrc) {
@@ -121,23 +114,16 @@ __global__ void stage_image_kernel(const uint8_t* __restrict__ units, const uint
       const int64_t r = u / g.nblk;
       const int b = (int)(u - r * g.nblk);
       const int64_t dr = gemv_image_row(r, half);
-      const int64_t tile = dr / (16 * g.R);
-      const int rr = (int)(dr - tile * 16 * g.R);
-      const int slab = b / g.S, bb = b - slab * g.S;
-      const bool last = slab == g.nslab - 1;
-      uint8_t* dst = img + (size_t)tile * g.tile_bytes + (size_t)slab * g.stage_bytes + (size_t)rr * (last ? g.RS_last : g.RS) +
-                     (size_t)(last ? g.d_off_last : g.d_off) + (size_t)bb * 2;
-      *reinterpret_cast<uint16_t*>(dst) = dsrc[u];
+      *reinterpret_cast<uint16_t*>(img + (size_t)((dr >> 4) * g.nblk + b) * cell_bytes + 16 * g.ub + 2 * (dr & 15)) = dsrc[u];
     }
   }
 }
 
 struct GemvSeg {
-  const uint8_t* img;  // stage images, [tiles][tile_bytes]
+  const uint8_t* img;  // cells, [16-row groups][blocks]
   int type;
   int rows;            // image rows that hold data (SWIGLU: 2 x the projection's rows)
   int tiles;
-  int RS, RS_last, d_off, d_off_last;
   uint32_t stage_bytes, stage_bytes_last, tile_bytes;
 };
 
@@ -534,10 +520,10 @@ __device__ __forceinline__ void load_bfrag(int type, const ActImage& a, int blk,
   f.sx = a.sx[blk];
 }
 
-// pa / pb point at this block's unit in rows g / g + 8 of the stage.
-__device__ __forceinline__ void compute_q4(const uint8_t* pa, const uint8_t* pb, const BFrag& f, const LaneCtx& L, float& acc0,
-                                           float& acc1) {
-  const uint4 h0 = *reinterpret_cast<const uint4*>(pa), h1 = *reinterpret_cast<const uint4*>(pb);
+// ph: the block's cell + 16 g (where chunk 0 of row g lies); pq: this lane's eight bytes of row g and of the first 32 elements
+// (32 elements further: + 512; row g + 8: + 128 in both).
+__device__ __forceinline__ void compute_q4(const uint8_t* ph, const uint8_t* pq, const BFrag& f, const LaneCtx& L, float& acc0, float& acc1) {
+  const uint4 h0 = *reinterpret_cast<const uint4*>(ph), h1 = *reinterpret_cast<const uint4*>(ph + 128);
   // eight 6-bit scales and minima per row, four to a word (get_scale_min_k4 of the reference,
   // quantization.cpp:145-155, applied to four sub-blocks at once)
   const uint32_t scA0 = h0.y & 0x3F3F3F3Fu, mnA0 = h0.z & 0x3F3F3F3Fu;
@@ -549,7 +535,7 @@ __device__ __forceinline__ void compute_q4(const uint8_t* pa, const uint8_t* pb,
   int Jlo0 = 0, Jlo1 = 0, Jhi0 = 0, Jhi1 = 0;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    const uint2 qa = *reinterpret_cast<const uint2*>(pa + 16 + 32 * c + 8 * L.t), qb = *reinterpret_cast<const uint2*>(pb + 16 + 32 * c + 8 * L.t);
+    const uint2 qa = *reinterpret_cast<const uint2*>(pq + 512 * c), qb = *reinterpret_cast<const uint2*>(pq + 512 * c + 128);
     int cl[4], ch[4];
     imma_16x8x32<false>(cl, qa.x & 0x0F0F0F0Fu, qb.x & 0x0F0F0F0Fu, qa.y & 0x0F0F0F0Fu, qb.y & 0x0F0F0F0Fu, f.b[2 * c].x, f.b[2 * c].y);
     imma_16x8x32<false>(ch, qa.x & 0xF0F0F0F0u, qb.x & 0xF0F0F0F0u, qa.y & 0xF0F0F0F0u, qb.y & 0xF0F0F0F0u, f.b[2 * c + 1].x,
@@ -570,17 +556,18 @@ __device__ __forceinline__ void compute_q4(const uint8_t* pa, const uint8_t* pb,
   acc1 = fmaf(f.sx, dm1.x * (L.wt * f1) - dm1.y * (L.wd * (float)M1), acc1);
 }
 
-__device__ __forceinline__ void compute_q6(const uint8_t* pa, const uint8_t* pb, float d0, float d1, const BFrag& f, const LaneCtx& L,
-                                           float& acc0, float& acc1) {
-  const uint4 sc0 = *reinterpret_cast<const uint4*>(pa + 192), sc1 = *reinterpret_cast<const uint4*>(pb + 192);
+__device__ __forceinline__ void compute_q6(const uint8_t* ph, const uint8_t* pq, const BFrag& f, const LaneCtx& L, float& acc0, float& acc1) {
+  const uint4 sc0 = *reinterpret_cast<const uint4*>(ph + 12 * 256), sc1 = *reinterpret_cast<const uint4*>(ph + 12 * 256 + 128);
+  const float d0 = half_bits_to_float(*reinterpret_cast<const uint16_t*>(ph + 16 * 208 - 14 * L.g));
+  const float d1 = half_bits_to_float(*reinterpret_cast<const uint16_t*>(ph + 16 * 208 + 16 - 14 * L.g));
   const uint32_t sw0[4] = {sc0.x, sc0.y, sc0.z, sc0.w}, sw1[4] = {sc1.x, sc1.y, sc1.z, sc1.w};
   int J0 = 0, J1 = 0;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const uint2 ha = *reinterpret_cast<const uint2*>(pa + 128 + 32 * h + 8 * L.t), hb = *reinterpret_cast<const uint2*>(pb + 128 + 32 * h + 8 * L.t);
+    const uint2 ha = *reinterpret_cast<const uint2*>(pq + 8 * 256 + 512 * h), hb = *reinterpret_cast<const uint2*>(pq + 8 * 256 + 512 * h + 128);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const uint2 la = *reinterpret_cast<const uint2*>(pa + 64 * h + 32 * q + 8 * L.t), lb = *reinterpret_cast<const uint2*>(pb + 64 * h + 32 * q + 8 * L.t);
+      const uint2 la = *reinterpret_cast<const uint2*>(pq + 512 * (2 * h + q)), lb = *reinterpret_cast<const uint2*>(pq + 512 * (2 * h + q) + 128);
 #pragma unroll
       for (int hi = 0; hi < 2; ++hi) {
         const int g4 = q + 2 * hi;  // 32-element group within the 128-element half (reference quantization.cpp:223-266)
@@ -607,14 +594,13 @@ __device__ __forceinline__ void compute_q6(const uint8_t* pa, const uint8_t* pb,
   acc1 = fmaf(f.sx * d1, L.wt * (float)J1 - 32.f * (L.wd * (float)C1), acc1);
 }
 
-__device__ __forceinline__ void compute_q8(const uint8_t* pa, const uint8_t* pb, const BFrag& f, const LaneCtx& L, float& acc0,
-                                           float& acc1) {
-  const uint4 da = *reinterpret_cast<const uint4*>(pa + 256), db = *reinterpret_cast<const uint4*>(pb + 256);
+__device__ __forceinline__ void compute_q8(const uint8_t* ph, const uint8_t* pq, const BFrag& f, const LaneCtx& L, float& acc0, float& acc1) {
+  const uint4 da = *reinterpret_cast<const uint4*>(ph + 16 * 256), db = *reinterpret_cast<const uint4*>(ph + 16 * 256 + 128);
   const uint32_t dw0[4] = {da.x, da.y, da.z, da.w}, dw1[4] = {db.x, db.y, db.z, db.w};
   float s0 = 0.f, s1 = 0.f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const uint2 qa = *reinterpret_cast<const uint2*>(pa + 32 * j + 8 * L.t), qb = *reinterpret_cast<const uint2*>(pb + 32 * j + 8 * L.t);
+    const uint2 qa = *reinterpret_cast<const uint2*>(pq + 512 * j), qb = *reinterpret_cast<const uint2*>(pq + 512 * j + 128);
     int c[4];
     imma_16x8x32<true>(c, qa.x, qb.x, qa.y, qb.y, f.b[j].x, f.b[j].y);
     // the scale field of a Q8_0 block is used by magnitude (reference quantization.cpp:85-87)
@@ -796,11 +782,11 @@ __device__ __forceinline__ void gemv_tiles(const GemvParams& prm, const GemvSeg&
                                            const LaneCtx& L, BFrag& bf) {
   GemvShared* sh = c.sh;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int ub = TYPE == T_Q4_K ? 144 : TYPE == T_Q6_K ? 208 : 272;
   const int nslab = prm.nslab;
-  // byte offset of this lane's first row (row g of the warp's row group) and block within a stage
-  const uint32_t off_full = (uint32_t)(c.rg * 16 + L.g) * (uint32_t)sg.RS + (uint32_t)c.bi * ub;
-  const uint32_t off_last = (uint32_t)(c.rg * 16 + L.g) * (uint32_t)sg.RS_last + (uint32_t)c.bi * ub;
+  // byte offsets of this warp's cell (+ row g) and of this lane's fragment within a stage (rows of several stages have one row
+  // group per tile); the fragments of Q4_K start at chunk 1
+  const uint32_t off_h = 16u * (uint32_t)L.g + (uint32_t)(c.rg * prm.S + c.bi) * (uint32_t)(TYPE == T_Q6_K ? 16 * 208 + 32 : TYPE == T_Q4_K ? 16 * 144 : 16 * 272);
+  const uint32_t off_q = off_h - 16u * (uint32_t)L.g + gemv_chunk(L.g, (TYPE == T_Q4_K ? 1 : 0) + (L.t >> 1)) + 8u * (uint32_t)(L.t & 1);
 #pragma unroll 1
   for (; c.tile < seg_end; c.tile += c.ncta, ++c.i) {
     float acc0 = 0.f, acc1 = 0.f;
@@ -816,20 +802,10 @@ __device__ __forceinline__ void gemv_tiles(const GemvParams& prm, const GemvSeg&
       }
       if (!pipe_aborted(sh) && !mbar_wait(&sh->full_bar[c.slot], c.use & 1)) pipe_fail(prm, sh);
       if (active) {
-        const int RSt = last ? sg.RS_last : sg.RS;
-        const uint8_t* pa = c.ring + (size_t)c.slot * prm.slot_bytes + (last ? off_last : off_full);
-        const uint8_t* pb = pa + 8 * RSt;
-        if (TYPE == T_Q4_K) {
-          compute_q4(pa, pb, bf, L, acc0, acc1);
-        } else if (TYPE == T_Q6_K) {
-          const uint8_t* ra = pa - c.bi * ub;
-          const int dof = (last ? sg.d_off_last : sg.d_off) + 2 * c.bi;
-          const float d0 = half_bits_to_float(*reinterpret_cast<const uint16_t*>(ra + dof));
-          const float d1 = half_bits_to_float(*reinterpret_cast<const uint16_t*>(ra + 8 * RSt + dof));
-          compute_q6(pa, pb, d0, d1, bf, L, acc0, acc1);
-        } else {
-          compute_q8(pa, pb, bf, L, acc0, acc1);
-        }
+        const uint8_t* slot = c.ring + (size_t)c.slot * prm.slot_bytes;
+        if (TYPE == T_Q4_K) compute_q4(slot + off_h, slot + off_q, bf, L, acc0, acc1);
+        else if (TYPE == T_Q6_K) compute_q6(slot + off_h, slot + off_q, bf, L, acc0, acc1);
+        else compute_q8(slot + off_h, slot + off_q, bf, L, acc0, acc1);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->empty_bar[c.slot]);  // this warp is done with the slot

@@ -113,6 +113,21 @@ def test_matmul_cut_tiles_and_token_tiles(pkg, name, rows, cols, tokens):
     assert np.abs(y - ref).max() <= 1e-3 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("name,rows,cols,batch", [("q4_k", 40, 256, 2), ("q6_k", 130, 512, 3), ("q8_0", 1000, 1792, 4), ("q4_k", 4100, 2048, 5), ("q6_k", 2500, 2304, 6),
+                                                  ("q8_0", 3000, 4096, 7), ("q4_k", 22016, 4096, 8), ("q4_k", 300, 4096, 15), ("q6_k", 4096, 11008, 5),
+                                                  ("q4_k", 200, 14336, 7), ("q4_k", 48, 28672, 3), ("q6_k", 40300, 4096, 6)])
+def test_matvec_batches(pkg, name, rows, cols, batch):
+    """Several vectors in one launch: odd and even numbers of them, one and several groups, one and several stages per tile, short
+    rows (several row groups per tile), rows of a length that leaves room for one vector only, many parked tiles."""
+    typ = TYPES[name]
+    blocks = pkg.synth.quantize(typ, pkg.synth.fill_normal(rows * cols, 93, rows + typ, 0.02))
+    wd = ol.dequant("oracle", typ, blocks).reshape(rows, cols)
+    x = pkg.synth.fill_normal(batch * cols, 94, cols, 1.0).reshape(batch, cols)
+    y = pkg.api.matvec(typ, blocks, rows, cols, x)
+    for b in range(batch):
+        assert rel_err(y[b], ol.matvec_f32("oracle", wd, x[b])) <= 1e-3
+
+
 def test_matvec_batch_and_edge_values(pkg):
     rows, cols = 8, 512
     w = pkg.synth.fill_normal(rows * cols, 5, 9, 0.02)

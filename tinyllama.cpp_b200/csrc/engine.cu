@@ -18,6 +18,7 @@
 #include "dense_gemm.cuh"
 #include "dequant.cuh"
 #include "gemv.cuh"
+#include "gemv_batch.cuh"
 #include "gemm_tc.cuh"
 #include "gguf.h"
 #include "latent_attn.cuh"
@@ -78,6 +79,10 @@ static void set_gemv_attrs() {
   const int maxb = GEMV_SMEM_BUDGET;
   CK(cudaFuncSetAttribute(gemv_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
   CK(cudaFuncSetAttribute(gemv_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
+  CK(cudaFuncSetAttribute(gemv_batch_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
+  CK(cudaFuncSetAttribute(gemv_batch_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
+  CK(cudaFuncSetAttribute(gemv_batch_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
+  CK(cudaFuncSetAttribute(gemv_batch_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
   CK(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX));
   (void)tensor_map_encoder();
   CK(cudaFuncSetAttribute((attn_decode_kernel<true, 0>), cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
@@ -266,6 +271,58 @@ static GemvSeg seg_of(const DevTensor& t) {
   return s;
 }
 
+// A launch that may start while the one before it runs (the kernel waits for it with griddepcontrol.wait).
+template <typename... P, typename... A>
+static void launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  CK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
+// Bytes the producer requests before the consumers hold their input vector (B200_GEMV_EARLY_KB, default 80).
+static size_t gemv_early_bytes() {
+  static const int kb = [] { const char* v = getenv("B200_GEMV_EARLY_KB"); return v && atoi(v) > 0 ? atoi(v) : 80; }();
+  return (size_t)kb * 1024;
+}
+
+// Several vectors on the batched kernel (gemv_batch.cuh), when its shared memory holds two of them and two ring slots (rows of
+// up to about 22000 elements); false: not this launch. The vectors are shared out evenly over as few CTAs as that
+// allows. 24-bit activations on one GPU only: the tensor-parallel exchange is built into the one-vector kernel.
+static bool launch_gemv_batch(const b200_engine* e, GemvParams p, int batch, cudaStream_t st, int* grid) {
+  if (batch < 2 || e->P != 3 || p.x_parts || p.epi == EPI_PEER || p.amax_peer[0]) return false;
+  const GvbGeom g = gvb_geometry(p.nblk);
+  int cell = 0;
+  p.ntiles = 0;
+  for (int s = 0; s < p.nseg; ++s) {
+    cell = std::max(cell, gemv_cell_bytes(p.seg[s].type));
+    p.seg[s].tiles = ((p.seg[s].rows + 15) / 16 + g.R - 1) / g.R;
+    p.ntiles += p.seg[s].tiles;
+  }
+  p.slot_bytes = (uint32_t)((g.R * g.S * cell + 127) / 128 * 128);
+  int np = std::min(GVB_MAX, batch + 1) / 2;
+  while (np > 0 && gvb_ring_offset(p.K, np) + 2 * (size_t)p.slot_bytes > (size_t)GEMV_SMEM_BUDGET) --np;
+  if (np == 0) return false;
+  const int groups = (batch + 2 * np - 1) / (2 * np), per = (batch + groups - 1) / groups;
+  np = (per + 1) / 2;
+  const size_t ring_off = gvb_ring_offset(p.K, np);
+  const int gx = std::max(1, std::min(p.ntiles, e->num_sms));
+  const int nslots = (int)std::min<size_t>(std::min(GEMV_MAX_STAGES, std::max(2, (p.ntiles + gx - 1) / gx * g.nst)), (GEMV_SMEM_BUDGET - ring_off) / p.slot_bytes);
+  p.early_stages = std::max(1, std::min(nslots, (int)(gemv_early_bytes() / p.slot_bytes)));
+  p.error_flag = e->d_error;
+  void (*kernel)(GemvParams, int, int, int) = np == 1 ? gemv_batch_kernel<1> : np == 2 ? gemv_batch_kernel<2> : np == 3 ? gemv_batch_kernel<3> : gemv_batch_kernel<4>;
+  launch_pdl(e->use_pdl, kernel, dim3(gx, groups), dim3(GEMV_THREADS), ring_off + (size_t)nslots * p.slot_bytes, st, p, nslots, per, batch);
+  *grid = gx;
+  return true;
+}
+
 // Fills in the launch geometry (tiles, ring slot size and depth), and starts the kernel with one
 // persistent CTA per SM (fewer when there are fewer tiles), as a programmatic dependent launch
 // when the engine allows it. Returns the grid width.
@@ -273,13 +330,15 @@ static int launch_gemv(const b200_engine* e, GemvParams p, int batch, cudaStream
   if (p.K % 256) throw std::runtime_error("gemv: K must be a multiple of 256");
   const GemvGeom g0 = gemv_geometry(p.seg[0].type, p.K);
   p.nblk = g0.nblk; p.nslab = g0.nslab; p.S = g0.S; p.S_last = g0.S_last; p.R = g0.R;
+  if (p.epi == EPI_SWIGLU && p.nseg != 1) throw std::runtime_error("gemv: SwiGLU takes the combined gate+up image");
+  int grid = 0;
+  if (launch_gemv_batch(e, p, batch, st, &grid)) return grid;
   p.ntiles = 0;
   uint32_t slot = 0;
   for (int s = 0; s < p.nseg; ++s) {
     p.ntiles += p.seg[s].tiles;
     slot = std::max(slot, std::max(p.seg[s].stage_bytes, p.seg[s].stage_bytes_last));
   }
-  if (p.epi == EPI_SWIGLU && p.nseg != 1) throw std::runtime_error("gemv: SwiGLU takes the combined gate+up image");
   p.slot_bytes = (slot + 127) / 128 * 128;
   const int gx = std::max(1, std::min(p.ntiles, e->num_sms));
   const size_t ring_off = gemv_ring_offset(p.K, e->P);
@@ -288,9 +347,7 @@ static int launch_gemv(const b200_engine* e, GemvParams p, int batch, cudaStream
   // ring depth: what fits, but no more slots than this CTA will ever fill
   const int stages_per_cta = ((p.ntiles + gx - 1) / gx) * p.nslab;
   const int nstages = std::max(1, (int)std::min<size_t>(std::min(GEMV_MAX_STAGES, stages_per_cta), (budget - ring_off) / p.slot_bytes));
-  // bytes the producer requests before the consumers hold their input vector (B200_GEMV_EARLY_KB, default 80)
-  static const int early_kb = [] { const char* v = getenv("B200_GEMV_EARLY_KB"); return v && atoi(v) > 0 ? atoi(v) : 80; }();
-  p.early_stages = std::max(1, std::min(nstages, (int)((size_t)early_kb * 1024 / p.slot_bytes)));
+  p.early_stages = std::max(1, std::min(nstages, (int)(gemv_early_bytes() / p.slot_bytes)));
   p.error_flag = e->d_error;
   const size_t smem = ring_off + (size_t)nstages * p.slot_bytes;
   cudaLaunchConfig_t cfg{};
@@ -308,22 +365,6 @@ static int launch_gemv(const b200_engine* e, GemvParams p, int batch, cudaStream
   return gx;
 }
 
-
-// A launch that may start while the one before it runs (the kernel waits for it with griddepcontrol.wait).
-template <typename... P, typename... A>
-static void launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  CK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
-}
 
 // Starts the tensor-core matmul for T tokens (gemm_tc.cuh). x16: [T][K] fp16 activations.
 static void encode_map(CUtensorMap* tm, CUtensorMapDataType dt, int rank, const void* base, const cuuint64_t* gdim, const cuuint64_t* gstr,

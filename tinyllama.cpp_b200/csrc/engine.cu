@@ -535,7 +535,7 @@ static int launch_linear(b200_engine* e, GemvParams p, int batch, cudaStream_t s
   launch_gemm_tc(e, t, st);
   int n = 2;
   if (p.amax_val) {  // lm_head: the matvec kernel leaves argmax partials; here a small kernel scans the logits
-    argmax_rows_kernel<<<batch, 256, 0, st>>>(p.y, p.y_stride, p.amax_row_offset, p.amax_val, p.amax_idx);
+    argmax_rows_kernel<<<batch, ARGMAX_THREADS, 0, st>>>(p.y, p.y_stride, p.amax_row_offset, p.amax_val, p.amax_idx);
     CK(cudaGetLastError());
     if (grid_out) *grid_out = 1;
     ++n;

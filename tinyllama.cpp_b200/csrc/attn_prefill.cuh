@@ -29,7 +29,8 @@ struct PrefillAttnParams {
   const float* v_scale;
   int slot, start, T;  // tokens occupy positions start .. start+T-1
   int nq, nkv, max_ctx;
-  float* out;  // [T][out_stride]
+  float* out;     // [T][out_stride], or
+  __half* out16;  // the same in fp16, the output projection's operand; one of the two
   int out_stride;
   float att_scale;
 };
@@ -271,14 +272,24 @@ __global__ void __launch_bounds__(PFA_THREADS, 2) attn_prefill_kernel(const Pref
   l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
   const float inv0 = 1.0f / (l0 + 1e-9f), inv1 = 1.0f / (l1 + 1e-9f);  // softmax_vector_cpu (utils.cpp:675-698)
   if (r0 < prm.T) {
-    float* dst = prm.out + (size_t)r0 * prm.out_stride + h * HD + 2 * t;
+    const size_t at = (size_t)r0 * prm.out_stride + h * HD + 2 * t;
+    if (prm.out16) {
 #pragma unroll
-    for (int i = 0; i < NT_O; ++i) *reinterpret_cast<float2*>(dst + i * 8) = make_float2(o[i][0] * inv0, o[i][1] * inv0);
+      for (int i = 0; i < NT_O; ++i) *reinterpret_cast<uint32_t*>(prm.out16 + at + i * 8) = pfa_pack(o[i][0] * inv0, o[i][1] * inv0);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NT_O; ++i) *reinterpret_cast<float2*>(prm.out + at + i * 8) = make_float2(o[i][0] * inv0, o[i][1] * inv0);
+    }
   }
   if (r1 < prm.T) {
-    float* dst = prm.out + (size_t)r1 * prm.out_stride + h * HD + 2 * t;
+    const size_t at = (size_t)r1 * prm.out_stride + h * HD + 2 * t;
+    if (prm.out16) {
 #pragma unroll
-    for (int i = 0; i < NT_O; ++i) *reinterpret_cast<float2*>(dst + i * 8) = make_float2(o[i][2] * inv1, o[i][3] * inv1);
+      for (int i = 0; i < NT_O; ++i) *reinterpret_cast<uint32_t*>(prm.out16 + at + i * 8) = pfa_pack(o[i][2] * inv1, o[i][3] * inv1);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NT_O; ++i) *reinterpret_cast<float2*>(prm.out + at + i * 8) = make_float2(o[i][2] * inv1, o[i][3] * inv1);
+    }
   }
 }
 

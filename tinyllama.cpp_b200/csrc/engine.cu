@@ -527,13 +527,14 @@ static int launch_linear(b200_engine* e, GemvParams p, int batch, cudaStream_t s
     return 1;
   }
   __half* x16 = static_cast<__half*>(x16_buf ? x16_buf : e->d_x16);
-  launch_pdl(e->use_pdl, to_half_kernel, dim3(batch), dim3(TOH_THREADS), 0, st, p.x, p.x_stride, p.norm_w, p.eps, p.K, x16);
+  if (p.x16) x16 = static_cast<__half*>(const_cast<void*>(p.x16));
+  else launch_pdl(e->use_pdl, to_half_kernel, dim3(batch), dim3(TOH_THREADS), 0, st, p.x, p.x_stride, p.norm_w, p.eps, p.K, x16);
   TcParams t{};
   for (int s = 0; s < p.nseg; ++s) t.seg[s] = p.seg[s];
-  t.nseg = p.nseg; t.K = p.K; t.x16 = x16; t.T = batch; t.epi = p.epi; t.y = p.y; t.y_stride = p.y_stride; t.y2 = p.y2;
+  t.nseg = p.nseg; t.K = p.K; t.x16 = x16; t.T = batch; t.epi = p.epi; t.y = p.y; t.y16 = static_cast<__half*>(p.y16); t.y_stride = p.y_stride; t.y2 = p.y2;
   t.y2_stride = p.y2_stride; t.resid = p.resid; t.rope = p.rope; t.positions = p.positions; t.head_dim = p.head_dim; t.max_pos = p.max_pos;
   launch_gemm_tc(e, t, st);
-  int n = 2;
+  int n = p.x16 ? 1 : 2;
   if (p.amax_val) {  // lm_head: the matvec kernel leaves argmax partials; here a small kernel scans the logits
     argmax_rows_kernel<<<batch, ARGMAX_THREADS, 0, st>>>(p.y, p.y_stride, p.amax_row_offset, p.amax_val, p.amax_idx);
     CK(cudaGetLastError());
@@ -646,12 +647,14 @@ static int packed_forward_step(b200_engine* e, int batch, int nsplit, cudaStream
       p.K = H; p.x = e->d_h; p.x_stride = H; p.norm_w = w.ffn_norm.f32(); p.eps = eps; p.epi = EPI_SWIGLU;
       if (peer) as_consumer(p);
       p.y = e->d_act; p.y_stride = F;
+      if (use_tc) p.y16 = e->d_act;
       p.trace = trace_rec(e, launches);
       launches += launch_linear(e, p, batch, st, use_tc);
     }
     {
       GemvParams p{};
       p.seg[0] = seg_of(w.wdown); p.nseg = 1; p.K = F; p.x = e->d_act; p.x_stride = F; p.epi = tp ? EPI_STORE : EPI_RESID;
+      if (use_tc) p.x16 = e->d_act;
       p.y = tp ? e->d_partial : e->d_h; p.y_stride = H;
       if (peer) as_producer(p, 2 * l + 1);
       p.trace = trace_rec(e, launches);
@@ -796,7 +799,7 @@ static void prefill_chunk(b200_engine* e, int T, const std::vector<int>& meta, c
         a.q = e->pf_q + (size_t)r.row0 * e->Hq; a.q_stride = e->Hq;
         a.k_cache = w.k_cache; a.v_cache = w.v_cache; a.k_scale = w.k_scale; a.v_scale = w.v_scale;
         a.slot = r.slot; a.start = r.start; a.T = r.len; a.nq = e->nq; a.nkv = e->nkv; a.max_ctx = e->max_ctx;
-        a.out = e->pf_attn + (size_t)r.row0 * e->Hq; a.out_stride = e->Hq; a.att_scale = 1.0f / std::sqrt((float)e->hd);
+        a.out16 = reinterpret_cast<__half*>(e->pf_attn) + (size_t)r.row0 * e->Hq; a.out_stride = e->Hq; a.att_scale = 1.0f / std::sqrt((float)e->hd);
         launch_prefill_attention(a, i8, e->hd, st);
       }
     } else {
@@ -812,7 +815,9 @@ static void prefill_chunk(b200_engine* e, int T, const std::vector<int>& meta, c
     }
     {
       GemvParams p{};
-      p.seg[0] = seg_of(w.wo); p.nseg = 1; p.K = e->Hq; p.x = e->pf_attn; p.x_stride = e->Hq; p.epi = tp ? EPI_STORE : EPI_RESID;
+      p.seg[0] = seg_of(w.wo); p.nseg = 1; p.K = e->Hq; p.x = e->pf_attn; p.x_stride = e->Hq;
+      if (prefill_attn_available(e->hd)) p.x16 = e->pf_attn;  // the attention kernel wrote fp16
+      p.epi = tp ? EPI_STORE : EPI_RESID;
       p.y = tp ? e->pf_partial : e->pf_h; p.y_stride = H;
       launch_linear(e, p, T, st, true, nullptr, e->pf_x16);
       if (tp) tp_reduce_add(e, T, st, e->pf_h, e->pf_partial);
@@ -821,12 +826,12 @@ static void prefill_chunk(b200_engine* e, int T, const std::vector<int>& meta, c
       GemvParams p{};
       p.seg[0] = seg_of(w.wgu); p.nseg = 1;
       p.K = H; p.x = e->pf_h; p.x_stride = H; p.norm_w = w.ffn_norm.f32(); p.eps = eps; p.epi = EPI_SWIGLU;
-      p.y = e->pf_act; p.y_stride = F;
+      p.y = e->pf_act; p.y16 = e->pf_act; p.y_stride = F;
       launch_linear(e, p, T, st, true, nullptr, e->pf_x16);
     }
     {
       GemvParams p{};
-      p.seg[0] = seg_of(w.wdown); p.nseg = 1; p.K = F; p.x = e->pf_act; p.x_stride = F; p.epi = tp ? EPI_STORE : EPI_RESID;
+      p.seg[0] = seg_of(w.wdown); p.nseg = 1; p.K = F; p.x16 = e->pf_act; p.epi = tp ? EPI_STORE : EPI_RESID;
       p.y = tp ? e->pf_partial : e->pf_h; p.y_stride = H;
       launch_linear(e, p, T, st, true, nullptr, e->pf_x16);
       if (tp) tp_reduce_add(e, T, st, e->pf_h, e->pf_partial);

@@ -57,6 +57,7 @@ struct TcParams {
   int NT;                         // tokens per tile: a multiple of 32, <= 256
   int epi;                        // EPI_STORE / EPI_RESID / EPI_QKV_ROPE / EPI_SWIGLU
   float* y;                       // [T][y_stride]
+  __half* y16;                    // SWIGLU: the next matmul's operand, in place of y (the rounding to_half_kernel would apply)
   int y_stride;
   float* y2;                      // QKV: new K then V rows, [T][y2_stride]
   int y2_stride;
@@ -418,11 +419,15 @@ __device__ __forceinline__ void tc_finish8(const TcParams& p, const TcWork& w, i
   if (p.epi == EPI_SWIGLU) {
     // image rows: eight gate rows then the same eight up rows (reference model.cpp:734-735, batch form
     // cpu_batch_processor.cpp:252-256: (g / (1 + exp(-g))) * u)
-    float* y = p.y + (size_t)t * p.y_stride + (row >> 4) * 8 + (row & 7);
+    const size_t at = (size_t)t * p.y_stride + (row >> 4) * 8 + (row & 7);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float up = __shfl_sync(0xffffffffu, v[j], (lane & 23) + 8);
-      if (row_ok && !(row & 8) && j < n) y[(size_t)j * p.y_stride] = (v[j] / (1.0f + expf(-v[j]))) * up;
+      if (row_ok && !(row & 8) && j < n) {
+        const float o = (v[j] / (1.0f + expf(-v[j]))) * up;
+        if (p.y16) p.y16[at + (size_t)j * p.y_stride] = __float2half_rn(o);
+        else p.y[at + (size_t)j * p.y_stride] = o;
+      }
     }
   } else if (p.epi == EPI_RESID) {
     if (!row_ok) return;

@@ -138,6 +138,8 @@ struct GemvParams {
   int x_stride;
   const float* norm_w;  // RMSNorm weight fused into the prologue, or nullptr
   float eps;
+  const void* x16;      // tensor-core matmul: the activations are there already in fp16, [batch][K]
+  void* y16;            // tensor-core matmul, SWIGLU: outputs in fp16, [batch][y_stride], instead of y
   int epi;
   float* y;             // STORE/RESID/SWIGLU: [batch][y_stride]; QKV: q output [batch][y_stride]
   int y_stride;

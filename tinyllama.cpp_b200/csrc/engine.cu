@@ -9,6 +9,7 @@
 #include <cstring>
 #include <functional>
 #include <memory>
+#include <system_error>
 #include <thread>
 
 #include "attn.cuh"

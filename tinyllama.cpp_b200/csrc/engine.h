@@ -73,7 +73,7 @@ struct b200_engine {
   b200::BlockModel* blocks = nullptr;  // set: a block model (layers above stay empty)
   float* rope = nullptr;
   // step buffers
-  int* d_tokens = nullptr;
+  int* d_tokens = nullptr;      // tokens | positions | slots (max_seqs each) | step counter | forced steps: one block, written by one copy
   int* d_positions = nullptr;
   int* d_slots = nullptr;
   int* d_argmax = nullptr;
@@ -124,6 +124,7 @@ struct b200_engine {
   std::map<int, b200::StepGraph> graphs;
   int64_t weight_bytes = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t landed[8] = {nullptr};  // pieces of logits that have reached h_logits_pinned
   std::vector<void*> allocations;
   // Load-time staging: host bytes reach the device through two pinned buffers (the copy of one chunk
   // overlaps the host-side memcpy of the next) into device scratch that is reused from tensor to tensor;

@@ -62,12 +62,19 @@ struct DgmShared {
 // kind::f16 with bfloat16 operands: D = F32, A and B = BF16 and K-major
 __host__ __device__ __forceinline__ uint32_t dgm_idesc(int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24); }
 
-__device__ __forceinline__ bool dgm_wait(const DgmParams& p, DgmShared* sh, void* bar, uint32_t parity) {
+__device__ __noinline__ bool dgm_wait_slow(const DgmParams& p, DgmShared* sh, void* bar, uint32_t parity) {
   if (*(volatile int*)&sh->abort_flag) return false;
   if (mbar_wait(bar, parity)) return true;
   *(volatile int*)&sh->abort_flag = 1;
   if (p.error_flag) *reinterpret_cast<volatile int*>(p.error_flag) = 1;
   return false;
+}
+__device__ __forceinline__ bool dgm_wait(const DgmParams& p, DgmShared* sh, void* bar, uint32_t parity) {
+  return mbar_try(bar, parity) ? true : dgm_wait_slow(p, sh, bar, parity);
+}
+// the same for a whole warp, with one answer
+__device__ __forceinline__ bool dgm_wait_warp(const DgmParams& p, DgmShared* sh, void* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, dgm_wait(p, sh, bar, parity)) != 0;
 }
 
 // this warp's 32 TMEM lanes, 16 consecutive columns
@@ -144,7 +151,7 @@ __device__ __forceinline__ DgmUnit dgm_unit(const DgmParams& p, int u) {
 }
 
 // grid = min(units, SMs)
-__global__ void __launch_bounds__(DGM_THREADS, 1) dense_gemm_kernel(const DgmParams p, const __grid_constant__ DgmMaps maps) {
+__global__ void __launch_bounds__(DGM_THREADS, 1) dense_gemm_kernel(const __grid_constant__ DgmParams p, const __grid_constant__ DgmMaps maps) {
   extern __shared__ uint8_t dgm_smem_raw[];
   __shared__ DgmShared sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -165,50 +172,60 @@ __global__ void __launch_bounds__(DGM_THREADS, 1) dense_gemm_kernel(const DgmPar
   const uint32_t tmem = sh.tmem_base;
 
   if (warp == DGM_EPI_WARPS) {
-    // ---- producer lane ----
-    if (lane == 0) {
-      int s = 0, st = 0;
-      uint32_t ph = 1;  // a fresh ring's slots count as empty
-      bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        const DgmUnit w = dgm_unit(p, u);
-        for (int k = 0; k < w.steps; ++k) {
-          if (s >= p.stages && !(ok = dgm_wait(p, &sh, &sh.empty[st], ph))) break;
-          uint8_t* a = smem + (size_t)st * stage_bytes;
+    // ---- producer warp: both serial roles run as whole warps with one elected lane for the copies and the MMAs (as a
+    //      branch for one lane the MMA role took several hundred cycles a step, see gemm_tc.cuh) ----
+    const uint32_t leader = warp_leader();
+    int s = 0, st = 0;
+    uint32_t ph = 1;  // a fresh ring's slots count as empty
+    bool ok = true;
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const DgmUnit w = dgm_unit(p, u);
+#pragma unroll 1
+      for (int k = 0; k < w.steps; ++k) {
+        if (s >= p.stages && !(ok = dgm_wait_warp(p, &sh, &sh.empty[st], ph))) break;
+        uint8_t* a = smem + (size_t)st * stage_bytes;
+        ++s;
+        if (leader) {
           mbar_expect_tx(&sh.full[st], stage_bytes);
-          tc_tma_load_2d(a, &maps.w[w.seg], (w.k0 + k) * TC_KC, w.row0, &sh.full[st]);
-          tc_tma_load_2d(a + TC_M * 128, &maps.x[w.seg], (w.k0 + k) * TC_KC, w.t0, &sh.full[st]);
-          sh.issued = ++s;
-          if (++st == p.stages) { st = 0; ph ^= 1u; }
+          *(volatile int*)&sh.issued = s;
         }
+        __syncwarp();
+        tc_tma_load_2d(leader, a, &maps.w[w.seg], (w.k0 + k) * TC_KC, w.row0, &sh.full[st]);
+        tc_tma_load_2d(leader, a + TC_M * 128, &maps.x[w.seg], (w.k0 + k) * TC_KC, w.t0, &sh.full[st]);
+        if (++st == p.stages) { st = 0; ph ^= 1u; }
       }
     }
     __syncwarp();
   } else if (warp == DGM_EPI_WARPS + 1) {
-    // ---- MMA lane ----
-    if (lane == 0) {
-      const uint32_t idesc = dgm_idesc(p.NT);
-      int st = 0, n = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++n) {
-        const DgmUnit w = dgm_unit(p, u);
-        const int buf = n & 1;
-        if (n >= 2 && !(ok = dgm_wait(p, &sh, &sh.acc_empty[buf], (uint32_t)((n / 2 - 1) & 1)))) break;
+    // ---- MMA warp ----
+    const uint32_t leader = warp_leader();
+    const uint32_t idesc = dgm_idesc(p.NT);
+    const uint64_t ad0 = tc_smem_desc(smem_u32(smem)), bd0 = tc_smem_desc(smem_u32(smem + TC_M * 128)), step = (uint64_t)(stage_bytes >> 4);
+    uint64_t ad = ad0, bd = bd0;
+    int st = 0, n = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++n) {
+      const DgmUnit w = dgm_unit(p, u);
+      const int buf = n & 1;
+      if (n >= 2 && !(ok = dgm_wait_warp(p, &sh, &sh.acc_empty[buf], (uint32_t)((n / 2 - 1) & 1)))) break;
+      const uint32_t d = tmem + (uint32_t)(buf * p.acc_cols);
+      uint32_t accumulate = 0;
+#pragma unroll 1
+      for (int k = 0; k < w.steps; ++k) {
+        if (!(ok = dgm_wait_warp(p, &sh, &sh.full[st], ph))) break;
         tc_fence_after();
-        const uint32_t d = tmem + (uint32_t)(buf * p.acc_cols);
-        for (int k = 0; k < w.steps; ++k) {
-          if (!(ok = dgm_wait(p, &sh, &sh.full[st], ph))) break;
-          tc_fence_after();
-          const uint32_t a = smem_u32(smem + (size_t)st * stage_bytes);
-          const uint64_t ad = tc_smem_desc(a), bd = tc_smem_desc(a + TC_M * 128);
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) tc_mma_f16(d, ad + 2 * k4, bd + 2 * k4, idesc, (k | k4) ? 1u : 0u);
-          tc_commit(&sh.empty[st]);
-          if (++st == p.stages) { st = 0; ph ^= 1u; }
-        }
-        if (ok) tc_commit(&sh.acc_full[buf]);
+        tc_mma_f16(leader, d, ad, bd, idesc, accumulate);
+        tc_mma_f16(leader, d, ad + 2, bd + 2, idesc, 1u);
+        tc_mma_f16(leader, d, ad + 4, bd + 4, idesc, 1u);
+        tc_mma_f16(leader, d, ad + 6, bd + 6, idesc, 1u);
+        accumulate = 1u;
+        tc_commit_if(leader, &sh.empty[st]);
+        ad += step;
+        bd += step;
+        if (++st == p.stages) { st = 0; ph ^= 1u; ad = ad0; bd = bd0; }
       }
+      if (ok) tc_commit_if(leader, &sh.acc_full[buf]);
     }
     __syncwarp();
   } else {

@@ -84,17 +84,18 @@ __device__ __forceinline__ void tc_dealloc(uint32_t taddr, int ncols) {  // the 
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 16 fp16 per instruction
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[smem] * B[smem]^T, M = 128, K = 16 16-bit elements per instruction. The whole warp calls it, the leader issues it:
+// control flow and addresses stay uniform over the warp (uniform registers, which the instruction wants)
+__device__ __forceinline__ void tc_mma_f16(uint32_t leader, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
-// the same with A in tensor memory: lane = row, each 32-bit column two consecutive elements along K. The whole warp calls it,
-// the leader issues it: control flow and addresses stay uniform over the warp (uniform registers, which the instruction wants)
+// the same with A in tensor memory: lane = row, each 32-bit column two consecutive elements along K
 __device__ __forceinline__ void tc_mma_f16_ts(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
@@ -104,6 +105,7 @@ __device__ __forceinline__ void tc_mma_f16_ts(uint32_t leader, uint32_t tmem_d, 
       ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// arrives on the mbarrier once every MMA issued so far by the leader has completed
 __device__ __forceinline__ void tc_commit_if(uint32_t leader, void* bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
@@ -125,10 +127,6 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16])
                : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// arrives on the mbarrier once every MMA issued so far by this thread has completed
-__device__ __forceinline__ void tc_commit(void* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 // this warp's 32 TMEM lanes, 8 consecutive columns: thread = lane, registers = columns
 __device__ __forceinline__ void tc_ld8(uint32_t taddr, float (&v)[8]) {
   uint32_t r[8];
@@ -312,7 +310,7 @@ __device__ __noinline__ bool tc_wait_slow(const TcParams& p, TcShared* sh, void*
   if (p.error_flag) *reinterpret_cast<volatile int*>(p.error_flag) = 1;
   return false;
 }
-__device__ __forceinline__ bool tc_wait(const TcParams& p, TcShared* sh, void* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try(void* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -321,15 +319,21 @@ __device__ __forceinline__ bool tc_wait(const TcParams& p, TcShared* sh, void* b
       : "=r"(ok)
       : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
-  return ok ? true : tc_wait_slow(p, sh, bar, parity);
+  return ok != 0;
+}
+__device__ __forceinline__ bool tc_wait(const TcParams& p, TcShared* sh, void* bar, uint32_t parity) {
+  return mbar_try(bar, parity) ? true : tc_wait_slow(p, sh, bar, parity);
 }
 __device__ __forceinline__ void tc_workers_sync() { asm volatile("bar.sync 14, %0;" ::"n"(TC_WORKERS) : "memory"); }
 
-// 2-D tiled TMA load (64 elements along K x rows, 128-byte swizzle)
-__device__ __forceinline__ void tc_tma_load_2d(void* dst, const void* tmap, int c0, int c1, void* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-               "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-               : "memory");
+// 2-D tiled TMA load (64 elements along K x rows, 128-byte swizzle), issued by the leader of the warp
+__device__ __forceinline__ void tc_tma_load_2d(uint32_t leader, void* dst, const void* tmap, int c0, int c1, void* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(leader)
+      : "memory");
 }
 // 3-D tiled TMA load of an activation stage: steps x NT tokens x 64 elements, each step a tile in the 128-byte swizzle
 __device__ __forceinline__ void tc_tma_load_3d(void* dst, const void* tmap, int c0, int c1, int c2, void* bar) {

@@ -18,6 +18,10 @@
 //     waited for it; so the warp runs it together, with few waits, and one lane is elected for the MMAs alone;
 //   * after a unit's last step the sixteen warps read their TMEM lanes back (tcgen05.ld 32x32b: thread =
 //     weight row, registers = tokens) and run the matvec kernel's epilogues.
+// Measured, 7B Q4_K shapes: a step of 16 sequences 8.3 ms with one CTA per tile and the fp16 tile in shared memory, 4.7 ms now;
+// a 1024-token prompt 32.7 and 23.1 ms. With few tokens the bound is issue: about 370 instructions per thread and
+// block, byte permutes at half rate, 1650 cycles a block and warp beside 1240 of MMA issue, where HBM would need 800. With 256
+// tokens it is the activation tiles: 128 KB a block and SM from L2, at about 36 bytes a cycle.
 // The roles meet on mbarriers only. Every wait is bounded; on a give-up the kernel sets the error word,
 // waits for its copies, frees its tensor memory and returns.
 //

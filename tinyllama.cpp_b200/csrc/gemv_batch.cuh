@@ -9,7 +9,8 @@
 // What bounds it: instruction issue. One vector takes about 340 warp instructions per (16 rows, 256 elements), which is
 // 85 % of the issue slots at the rate HBM delivers the cell; one launch column per vector therefore took 5 x the time for 5
 // vectors (62 us a launch for 5 sequences of a 7B Q4_K model, 14 us for one). A further pair costs about 110 instructions
-// here (Q6_K: 180).
+// here (Q6_K: 180): 28 to 45 us a launch, 6.9 -> 4.4 ms for that model's step of 5 sequences over 600 tokens. (The integer
+// MMA itself is not the limit: 8.1 cycles per SM quarter.)
 //
 // Layout: the digit planes of all vectors of the CTA lie in shared memory (13.8 KB a vector at K = 4096, 37 KB at 11008) and
 // B fragments are read from there for each cell, not kept in registers. To leave room for a ring, a stage holds at most eight
@@ -470,8 +471,12 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_batch_kernel(const __gri
     return;
   }
   const int lane = threadIdx.x & 31;
+  unsigned long long* rec = (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ? prm.trace : nullptr;
+  trace_stamp(rec, 0);
   pdl_wait();
+  for (int i = 1; i < 5; ++i) trace_stamp(rec, i);
   gvb_build<NP>(prm, &sh, smem, first, nv);
+  trace_stamp(rec, 5);
   GvbLane G;
   G.L.g = lane >> 2;
   G.L.t = lane & 3;
@@ -495,6 +500,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_batch_kernel(const __gri
     else if (type == T_Q6_K) gvb_tiles<NP, T_Q6_K>(prm, &sh, smem, ring, nslots, g, G, seg_end, tile, i, n, first, nv);
     else gvb_tiles<NP, T_Q8_0>(prm, &sh, smem, ring, nslots, g, G, seg_end, tile, i, n, first, nv);
   }
+  trace_stamp(rec, 6);
   if (prm.amax_val) consumer_sync();  // all rows are in `best`
   if (prm.amax_val && threadIdx.x < nv) {
     const unsigned long long key = sh.best[threadIdx.x];
@@ -502,6 +508,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_batch_kernel(const __gri
     prm.amax_val[(size_t)(first + threadIdx.x) * gridDim.x + blockIdx.x] = key ? __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u) : -INFINITY;
     prm.amax_idx[(size_t)(first + threadIdx.x) * gridDim.x + blockIdx.x] = key ? (int)~(uint32_t)key : 0x7fffffff;
   }
+  trace_stamp(rec, 7);
 }
 
 }  // namespace b200

@@ -297,8 +297,13 @@ static size_t gemv_early_bytes() {
 // Several vectors on the batched kernel (gemv_batch.cuh), when its shared memory holds two of them and two ring slots (rows of
 // up to about 22000 elements); false: not this launch. The vectors are shared out evenly over as few CTAs as that
 // allows. 24-bit activations on one GPU only: the tensor-parallel exchange is built into the one-vector kernel.
+// Where one launch column per vector finds an SM for every tile at once, the columns cost no more than one vector and
+// stay: a step of 6 sequences of the toy model takes 107 us that way, 129 us with this kernel's longer prologue.
 static bool launch_gemv_batch(const b200_engine* e, GemvParams p, int batch, cudaStream_t st, int* grid) {
   if (batch < 2 || e->P != 3 || p.x_parts || p.epi == EPI_PEER || p.amax_peer[0]) return false;
+  int tiles = 0;
+  for (int s = 0; s < p.nseg; ++s) tiles += p.seg[s].tiles;
+  if ((long long)tiles * batch <= e->num_sms) return false;
   const GvbGeom g = gvb_geometry(p.nblk);
   int cell = 0;
   p.ntiles = 0;

@@ -1,0 +1,41 @@
+// Checks of csrc/host_copy.h: every byte of a buffer belongs to one piece, whatever its size.
+#include "host_copy.h"
+
+#include <cstdio>
+#include <vector>
+
+using namespace b200;
+
+static int failures = 0;
+#define CHECK(cond, ...) \
+  do { if (!(cond)) { ++failures; std::printf("line %d: %s: ", __LINE__, #cond); std::printf(__VA_ARGS__); std::printf("\n"); } } while (0)
+
+static void check_cover(size_t n, int pieces) {
+  const CopyPieces p(n, pieces);
+  size_t at = 0;
+  for (int i = 0; i < pieces; ++i) {
+    CHECK(p.begin(i) == at, "%zu bytes, %d pieces, piece %d", n, pieces, i);
+    at += p.size(i);
+  }
+  CHECK(at == n, "%zu bytes in %d pieces: %zu covered", n, pieces, at);
+}
+
+int main() {
+  for (int pieces : {1, 4, 8})
+    for (size_t pages : {0, 1, 7, 256, 2048})
+      for (int extra = -9; extra <= 9; ++extra) {
+        const long long n = (long long)pages * 4096 * pieces + extra;
+        if (n >= 0) check_cover((size_t)n, pieces);
+      }
+  // logits of 63 / 33 / 17 sequences whose number of values is one above a multiple of 8192
+  for (size_t n : {63 * (size_t)36799, 33 * (size_t)66529, 17 * (size_t)127217}) check_cover(4 * n, 8);
+
+  for (size_t n : {(size_t)100, ((size_t)8 << 20) - 1, ((size_t)8 << 20) + 1, ((size_t)8 << 20) + 4 * 4096 + 3}) {
+    std::vector<unsigned char> src(n), dst(n, 0);
+    for (size_t i = 0; i < n; ++i) src[i] = (unsigned char)(1 + i % 251);
+    parallel_memcpy(dst.data(), src.data(), n);
+    CHECK(src == dst, "%zu bytes", n);
+  }
+  std::printf("%d failures\n", failures);
+  return failures ? 1 : 0;
+}

@@ -5,6 +5,7 @@ over the root mean square of the logits. Limits: 1e-4 for a 32-bit engine; for a
 the operands of the matrix products to bfloat16 does to the plain model's logits of the same tokens.
 """
 import copy
+import ctypes
 import json
 import os
 import subprocess
@@ -422,6 +423,26 @@ def test_batches_of_unequal_requests_match_each_alone(pkg, case, name, dtype, ba
     tail = eng.prefill_batch([s[-1:] for s in seqs], slots=slots, start_pos=[n + 5 for n in lens])
     for i in range(batch):
         assert err(tail[i:i + 1], refs[i][-1:]) < limit
+
+
+def test_batch_over_a_large_odd_vocabulary(pkg, case):
+    """17 x 127217 logits: one value more than a whole number of pages in each of the eight pieces that they travel in. The caller's
+    buffer holds NaN before the call."""
+    batch, vocab = 17, 127217
+    assert batch * vocab % 8192 == 1
+    c = case("wide_vocab", cfg=bm.config([bm.wkv(heads=2, dim=16, rank=4, ff=0)], width=24, vocab=vocab))
+    eng = engine(pkg, c, "bfloat16", max_seqs=batch, max_ctx=16)
+    toks = np.asarray(bm.tokens(c.cfg, batch), np.int32)
+    pos = np.zeros(batch, np.int32)
+    logits, amax = np.full((batch, vocab), np.nan, np.float32), np.empty(batch, np.int32)
+    lib, ptr = pkg.api.lib(), lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    assert lib.b200_decode(eng._h, batch, ptr(toks), ptr(pos), None, ptr(logits), ptr(amax)) == 0
+    eng.close()
+    assert not np.isnan(logits).any()
+    assert np.array_equal(amax, logits.argmax(axis=1))
+    for b in range(batch):
+        t = [int(toks[b])]
+        assert err(logits[b:b + 1], c.plain(t)) < c.limit("bfloat16", t)
 
 
 @pytest.mark.parametrize("name", ["odd", "wkv_only", "piz_odd", "piz_wide"])

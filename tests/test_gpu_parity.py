@@ -5,6 +5,7 @@ Tolerances (stated here, used below):
   matvec                 |y - ref| <= 1e-3 * max(|ref_i|, 1e-3 * max|ref|)   (ref = Kahan FP32 dot, utils.cpp:349-397)
   logits                 <= 2e-2 absolute; greedy ids identical for 32 steps
 """
+import ctypes
 import os
 
 import numpy as np
@@ -422,6 +423,25 @@ def test_batch16_decode_takes_tensor_core_path(pkg, tiny_models, scheme, kv):
             nxt.append(int(ref.argmax()))
         toks, pos = nxt, [p + 1 for p in pos]
     eng.close()
+
+
+@pytest.mark.parametrize("vocab,batch", [(36798, 63), (20004, 17), (66532, 33)])
+def test_batch_decode_hands_over_large_vocabularies(pkg, tmp_path, vocab, batch):
+    """Logits that reach the caller in four or eight pieces (from 512 KB and 8 MB on), and their first maxima through the four-load and the one-load form of the argmax. The caller's
+    buffer holds NaN before the call. Tolerance of the logits: that of the fp16 matmul, as above."""
+    path = pkg.synth.write_gguf(str(tmp_path / "wide.gguf"), "tiny", scheme=1, vocab=vocab, n_layers=1, norm_random=True)
+    eng = pkg.Engine.from_gguf(path, max_seqs=batch, max_ctx=16)
+    toks = np.random.default_rng(vocab).integers(0, vocab, batch).astype(np.int32)
+    pos = np.zeros(batch, np.int32)
+    logits, amax = np.full((batch, vocab), np.nan, np.float32), np.empty(batch, np.int32)
+    lib, ptr = pkg.api.lib(), lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    assert lib.b200_decode(eng._h, batch, ptr(toks), ptr(pos), None, ptr(logits), ptr(amax)) == 0
+    eng.close()
+    assert not np.isnan(logits).any()
+    assert np.array_equal(amax, logits.argmax(axis=1))
+    orc = ol.OracleModel.from_gguf(path, max_seqs=batch)
+    for b in (0, batch // 2, batch - 1):
+        assert np.abs(logits[b] - orc.decode(int(toks[b]), 0, seq=b)).max() <= 2e-2
 
 
 @pytest.mark.parametrize("splits", [1, 3])

@@ -22,6 +22,7 @@
 #include "gemv_batch.cuh"
 #include "gemm_tc.cuh"
 #include "gguf.h"
+#include "host_copy.h"
 #include "latent_attn.cuh"
 #include "misc.cuh"
 #include "rglru.cuh"
@@ -39,19 +40,6 @@ static T* dev_alloc(b200_engine* e, size_t n) {
   CK(cudaMalloc(&p, std::max<size_t>(n * sizeof(T), 16)));
   if (e) e->allocations.push_back(p);
   return static_cast<T*>(p);
-}
-
-// memcpy split over a few threads: one thread moves 5-8 GB/s out of the page cache, which is less than the link takes.
-static void parallel_memcpy(void* dst, const void* src, size_t n) {
-  const int nt = n >= ((size_t)8 << 20) ? 4 : 1;
-  if (nt == 1) { std::memcpy(dst, src, n); return; }
-  std::thread th[4];
-  const size_t per = (n / nt + 4095) & ~(size_t)4095;
-  for (int i = 0; i < nt; ++i) {
-    const size_t off = std::min(n, per * i), len = std::min(per, n - off);
-    th[i] = std::thread([=] { if (len) std::memcpy(static_cast<uint8_t*>(dst) + off, static_cast<const uint8_t*>(src) + off, len); });
-  }
-  for (int i = 0; i < nt; ++i) th[i].join();
 }
 
 // cuTensorMapEncodeTiled, fetched from the driver at run time (the library links only the runtime).

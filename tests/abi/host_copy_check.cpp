@@ -1,6 +1,8 @@
-// Checks of csrc/host_copy.h: every byte of a buffer belongs to one piece, whatever its size.
+// Checks of csrc/host_copy.h: every byte of a buffer belongs to one piece, whatever its size, and pieces that may not be handed
+// over leave the destination alone.
 #include "host_copy.h"
 
+#include <atomic>
 #include <cstdio>
 #include <vector>
 
@@ -35,6 +37,17 @@ int main() {
     for (size_t i = 0; i < n; ++i) src[i] = (unsigned char)(1 + i % 251);
     parallel_memcpy(dst.data(), src.data(), n);
     CHECK(src == dst, "%zu bytes", n);
+  }
+  const size_t n = 8 * 4096 * 3 + 5;
+  std::vector<unsigned char> src(n, 7), untouched(n, 1);
+  for (int nt : {1, 4}) {
+    std::atomic<int> seen{0};
+    std::vector<unsigned char> dst(n, 1);
+    hand_over(dst.data(), src.data(), CopyPieces(n, 8), 8, nt, [&](int) { ++seen; return true; });
+    CHECK(dst == src && seen == 8, "%d threads, %d pieces asked for", nt, seen.load());
+    dst.assign(n, 1);
+    hand_over(dst.data(), src.data(), CopyPieces(n, 8), 8, nt, [](int) { return false; });
+    CHECK(dst == untouched, "%d threads, refused pieces", nt);
   }
   std::printf("%d failures\n", failures);
   return failures ? 1 : 0;

@@ -31,4 +31,25 @@ inline void parallel_memcpy(void* dst, const void* src, size_t n) {
   for (int i = 1; i < nt; ++i) th[i].join();
 }
 
+// Hands a buffer over piece by piece as it lands, on nt threads: piece i is copied once landed(i), which waits for it, says that
+// it may be (false: the destination keeps what it held).
+template <class Landed>
+inline void hand_over(void* dst, const void* src, const CopyPieces& p, int pieces, int nt, Landed landed) {
+  auto take = [&](int i) {
+    if (landed(i)) copy_piece(dst, src, p, i);
+  };
+  std::thread th[8];
+  for (int t = 1; t < nt; ++t) {
+    try {
+      th[t] = std::thread([&take, t, nt, pieces] { for (int i = t; i < pieces; i += nt) take(i); });
+    } catch (const std::system_error&) {
+      // no further thread to be had: its pieces are taken below
+    }
+  }
+  for (int i = 0; i < pieces; ++i)
+    if (i % nt == 0 || !th[i % nt].joinable()) take(i);
+  for (int t = 1; t < nt; ++t)
+    if (th[t].joinable()) th[t].join();
+}
+
 }  // namespace b200

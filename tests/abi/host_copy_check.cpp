@@ -1,9 +1,11 @@
 // Checks of csrc/host_copy.h: every byte of a buffer belongs to one piece, whatever its size, and pieces that may not be handed
-// over leave the destination alone.
+// over leave the destination alone; further threads enter before their first piece, and calls do without those that cannot be had.
 #include "host_copy.h"
 
 #include <atomic>
 #include <cstdio>
+#include <cstdlib>
+#include <new>
 #include <vector>
 
 using namespace b200;
@@ -11,6 +13,17 @@ using namespace b200;
 static int failures = 0;
 #define CHECK(cond, ...) \
   do { if (!(cond)) { ++failures; std::printf("line %d: %s: ", __LINE__, #cond); std::printf(__VA_ARGS__); std::printf("\n"); } } while (0)
+
+// Allocations of the main thread that still succeed (-1: all): what std::thread needs for its start-up state.
+static thread_local int allocations_left = -1;
+void* operator new(size_t n) {
+  if (allocations_left == 0) throw std::bad_alloc();
+  if (allocations_left > 0) --allocations_left;
+  if (void* p = std::malloc(n)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 
 static void check_cover(size_t n, int pieces) {
   const CopyPieces p(n, pieces);
@@ -39,15 +52,36 @@ int main() {
     CHECK(src == dst, "%zu bytes", n);
   }
   const size_t n = 8 * 4096 * 3 + 5;
-  std::vector<unsigned char> src(n, 7), untouched(n, 1);
+  const std::vector<unsigned char> src(n, 7), untouched(n, 1);
+  std::vector<unsigned char> dst;
   for (int nt : {1, 4}) {
     std::atomic<int> seen{0};
-    std::vector<unsigned char> dst(n, 1);
-    hand_over(dst.data(), src.data(), CopyPieces(n, 8), 8, nt, [&](int) { ++seen; return true; });
+    dst.assign(n, 1);
+    hand_over(dst.data(), src.data(), CopyPieces(n, 8), 8, nt, [] {}, [&](int) { ++seen; return true; });
     CHECK(dst == src && seen == 8, "%d threads, %d pieces asked for", nt, seen.load());
     dst.assign(n, 1);
-    hand_over(dst.data(), src.data(), CopyPieces(n, 8), 8, nt, [](int) { return false; });
+    hand_over(dst.data(), src.data(), CopyPieces(n, 8), 8, nt, [] {}, [](int) { return false; });
     CHECK(dst == untouched, "%d threads, refused pieces", nt);
+  }
+
+  // every further thread enters once, before its first piece; the calling one does not
+  static thread_local int entered = 0;
+  std::atomic<int> threads{0}, early{0};
+  const std::thread::id me = std::this_thread::get_id();
+  dst.assign(n, 1);
+  hand_over(dst.data(), src.data(), CopyPieces(n, 8), 8, 4, [&] { ++entered; ++threads; }, [&](int) {
+    if (entered != (std::this_thread::get_id() == me ? 0 : 1)) ++early;
+    return true;
+  });
+  CHECK(dst == src && threads == 3 && early == 0, "%d threads entered, %d pieces out of order", threads.load(), early.load());
+
+  // no memory for the second or third thread: its pieces are handed over all the same, and nothing is thrown
+  for (int left : {0, 1, 2}) {
+    dst.assign(n, 1);
+    allocations_left = left;
+    hand_over(dst.data(), src.data(), CopyPieces(n, 8), 8, 4, [] {}, [](int) { return true; });
+    allocations_left = -1;
+    CHECK(dst == src, "%d allocations", left);
   }
   std::printf("%d failures\n", failures);
   return failures ? 1 : 0;

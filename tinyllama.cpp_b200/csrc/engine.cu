@@ -9,8 +9,6 @@
 #include <cstring>
 #include <functional>
 #include <memory>
-#include <system_error>
-#include <thread>
 
 #include "attn.cuh"
 #include "attn_cluster.cuh"

@@ -149,6 +149,11 @@ int b200_dequant(int ggml_type, const void* host_blocks, size_t n_blocks, float*
  * matvec_f32_f32_cuda (cuda_kernels.cu:291-314) / matvec_*_f32_vector_cpu (utils.cpp:293-397). */
 int b200_matvec(int ggml_type, const void* host_blocks, int64_t rows, int64_t cols, const float* host_x,
                 int batch, int act_planes, float* host_y);
+/* Which kernel matvec launches that follow one another take on one GPU of num_sms SMs (host arithmetic, no GPU): per launch the
+ * vectors that a CTA of the several-vector kernel takes, or 0 for one launch column per vector. launches [n][7]: input dimension,
+ * then block type and rows (0: none) of up to three matrices. A decode step passes a layer's four launches (q/k/v; output
+ * projection; gate and up as one matrix of 2 x ffn rows; down) and its lm_head by itself; b200_matvec its one launch. */
+int b200_matvec_plan(int n, const int32_t* launches, int batch, int act_planes, int num_sms, int32_t* vectors_per_cta);
 /* Y[t][r] = dot(W[r,:], X[t,:]) for n_tokens rows of X on the tensor cores (tcgen05, fp16 operands, FP32
  * accumulation in tensor memory): the batch >= 16 / prompt path that replaces matmul_*_f32_batch_cpu
  * (utils.cpp:730-782, 890-1044) and smart_gemm_batch_cuda (model.cpp:2141-2249). host_x [n_tokens][cols],

@@ -80,3 +80,40 @@ def test_prefill_chunk_plan(pkg):
             else:
                 assert ends == -1
         assert seq == len(lens) and pos == 0
+
+
+def layer_launches(shape, qo=12, v=14, gate_up=12, down=14):
+    """The four launches of a layer as `matvec_plan` takes them."""
+    H, F = shape["hidden"], shape["ffn"]
+    kvd = H // shape["n_heads"] * shape["n_kv_heads"]
+    return [(H, [(qo, H), (qo, kvd), (v, kvd)]), (H, [(qo, H)]), (H, [(gate_up, 2 * F)]), (F, [(down, H)])]
+
+
+def test_matvec_plan(pkg):
+    """Which launches of a step of 2 to 15 sequences share their weights (gemv_batch.cuh, gvb_takes), on 148 SMs."""
+    plan, S = pkg.api.matvec_plan, pkg.synth.SHAPES
+    # a model whose launches all find an SM for every tile and vector stays with one column per vector, and so does one of up to
+    # two waves where a CTA would take seven or eight vectors (the step of 15 sequences of the 512-wide model)
+    for name in ("tiny", "tiny_mha"):
+        for batch in range(2, 16):
+            assert plan(layer_launches(S[name]), batch) == [0, 0, 0, 0], (name, batch)
+            assert plan([(S[name]["hidden"], [(14, S[name]["vocab"])])], batch) == [0]
+    # two sequences: a layer stays with one kernel, although its O projection's columns would fit
+    assert plan(layer_launches(S["tinyllama-1.1b"]), 2) == [2, 2, 2, 2]
+    assert plan([layer_launches(S["tinyllama-1.1b"])[1]], 2) == [0]
+    # more of them: launch by launch
+    w = dict(hidden=1024, ffn=2816, n_heads=16, n_kv_heads=4)
+    assert plan(layer_launches(w), 2) == [2, 2, 2, 2]
+    assert plan(layer_launches(w), 4) == [0, 0, 4, 4]
+    assert plan(layer_launches(w), 9) == [5, 0, 5, 5]
+    # 11008-element rows leave room for four vectors, 14336-element rows for two, 28672-element rows for none
+    assert plan(layer_launches(S["llama2-7b"]), 5) == [5, 5, 5, 3]
+    assert plan(layer_launches(S["llama3-8b"]), 8)[3] == 2
+    assert plan(layer_launches(S["llama2-70b"]), 8)[3] == 0
+    # one vector, 16-bit activations: never
+    assert plan(layer_launches(S["llama2-7b"]), 1) == [0] * 4
+    assert plan(layer_launches(S["llama2-7b"]), 5, planes=2) == [0] * 4
+    with pytest.raises(pkg.B200Error):
+        plan([(300, [(12, 64)])], 2)
+    with pytest.raises(pkg.B200Error):
+        plan([(256, [(3, 64)])], 2)

@@ -30,7 +30,7 @@ EXPORTS = [
     "b200_last_error", "b200_device_count", "b200_engine_create", "b200_engine_upload_tensor",
     "b200_engine_finalize", "b200_engine_load_gguf", "b200_engine_load_model", "b200_engine_get_desc", "b200_engine_destroy",
     "b200_kv_reset", "b200_lookup_embedding", "b200_forward", "b200_prefill", "b200_prefill_rows", "b200_prefill_batch", "b200_prefill_plan", "b200_decode",
-    "b200_generate_greedy", "b200_generate_greedy_penalized", "b200_dequant", "b200_matvec", "b200_matmul", "b200_rmsnorm", "b200_rmsnorm_batch",
+    "b200_generate_greedy", "b200_generate_greedy_penalized", "b200_dequant", "b200_matvec", "b200_matvec_plan", "b200_matmul", "b200_rmsnorm", "b200_rmsnorm_batch",
     "b200_fused_qkv_rope", "b200_fused_gate_up_swiglu", "b200_attention_decode", "b200_attention_prefill",
     "b200_attention_decode_noalloc", "b200_engine_stats", "b200_engine_time_kernel", "b200_engine_read_trace",
     "b200_nccl_unique_id", "b200_tp_share", "b200_selftest_exchange_timeout"]
@@ -64,6 +64,7 @@ def lib():
     L.b200_prefill_rows.argtypes = [_vp, _i, _vp, _i, _i, _vp, _i, _vp]
     L.b200_decode.argtypes = [_vp, _i, _vp, _vp, _vp, _vp, _vp]
     L.b200_prefill_batch.argtypes = [_vp, _i, _vp, _vp, _vp, _vp, _vp]
+    L.b200_matvec_plan.argtypes = [_i, _vp, _i, _i, _i, _vp]
     L.b200_prefill_plan.argtypes = [_i, _vp, _i, _vp, _i, ctypes.POINTER(_i)]
     L.b200_generate_greedy.argtypes = [_vp, _i, _vp, _vp, _vp, _i, _vp, ctypes.POINTER(ctypes.c_float)]
     L.b200_generate_greedy_penalized.argtypes = [_vp, _i, _vp, _vp, _vp, _i, ctypes.c_float, _vp, _vp, _vp, ctypes.POINTER(ctypes.c_float)]
@@ -280,6 +281,17 @@ def matvec(ggml_type, blocks, rows, cols, x, act_planes=3):
     y = np.empty((batch, rows), np.float32)
     _check(lib().b200_matvec(ggml_type, _ptr(blocks), rows, cols, _ptr(x), batch, act_planes, _ptr(y)))
     return y[0] if x.ndim == 1 else y
+
+
+def matvec_plan(launches, batch, planes=3, num_sms=148):
+    """Vectors per CTA of the several-vector kernel (0: one launch column per vector) for matvec launches that follow one
+    another; a launch is (input dimension, [(block type, rows), ...])."""
+    table = np.zeros((len(launches), 7), np.int32)
+    for row, (cols, mats) in zip(table, launches):
+        row[:1 + 2 * len(mats)] = [cols] + [v for m in mats for v in m]
+    out = np.empty(len(launches), np.int32)
+    _check(lib().b200_matvec_plan(len(launches), _ptr(table), batch, planes, num_sms, _ptr(out)))
+    return out.tolist()
 
 
 def matmul(ggml_type, blocks, rows, cols, x):

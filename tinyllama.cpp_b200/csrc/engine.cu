@@ -280,37 +280,44 @@ static size_t gemv_early_bytes() {
   return (size_t)kb * 1024;
 }
 
-// Several vectors on the batched kernel (gemv_batch.cuh), when its shared memory holds two of them and two ring slots (rows of
-// up to about 22000 elements); false: not this launch. The vectors are shared out evenly over as few CTAs as that
-// allows. 24-bit activations on one GPU only: the tensor-parallel exchange is built into the one-vector kernel.
-// Where one launch column per vector finds an SM for every tile at once, the columns cost no more than one vector and
-// stay: a step of 6 sequences of the toy model takes 107 us that way, 129 us with this kernel's longer prologue.
-static bool launch_gemv_batch(const b200_engine* e, GemvParams p, int batch, cudaStream_t st, int* grid) {
-  if (batch < 2 || e->P != 3 || p.x_parts || p.epi == EPI_PEER || p.amax_peer[0]) return false;
-  int tiles = 0;
-  for (int s = 0; s < p.nseg; ++s) tiles += p.seg[s].tiles;
-  if ((long long)tiles * batch <= e->num_sms) return false;
+static GvbLaunch gvb_launch(int K, const GemvSeg* seg, int nseg) {
+  GvbLaunch l{K, 0, 0};
+  for (int s = 0; s < nseg; ++s) {
+    l.tiles += seg[s].tiles;
+    l.cell = std::max(l.cell, gemv_cell_bytes(seg[s].type));
+  }
+  return l;
+}
+
+// Launches of a step that follow one another, and which of them a call is about.
+struct GvbPlace {
+  const GvbLaunch* launches;
+  int n, i;
+};
+
+// Several vectors on the batched kernel (gemv_batch.cuh) if gvb_takes says so; false: not this launch. place: the launch among its
+// neighbours (nullptr: by itself). 24-bit activations on one GPU only: the tensor-parallel exchange is built into the one-vector
+// kernel, and the step of a tensor-parallel engine stays with it throughout.
+static bool launch_gemv_batch(const b200_engine* e, GemvParams p, int batch, cudaStream_t st, const GvbPlace* place, int* grid) {
+  if (batch < 2 || e->P != 3 || e->tp_size > 1 || p.x_parts) return false;
+  const GvbLaunch self = gvb_launch(p.K, p.seg, p.nseg);
+  if (!(place ? gvb_takes(place->launches, place->n, place->i, batch, e->num_sms) : gvb_takes(&self, 1, 0, batch, e->num_sms))) return false;
+  const GvbSplit split = gvb_split(self, batch);
   const GvbGeom g = gvb_geometry(p.nblk);
-  int cell = 0;
   p.ntiles = 0;
   for (int s = 0; s < p.nseg; ++s) {
-    cell = std::max(cell, gemv_cell_bytes(p.seg[s].type));
     p.seg[s].tiles = ((p.seg[s].rows + 15) / 16 + g.R - 1) / g.R;
     p.ntiles += p.seg[s].tiles;
   }
-  p.slot_bytes = (uint32_t)((g.R * g.S * cell + 127) / 128 * 128);
-  int np = std::min(GVB_MAX, batch + 1) / 2;
-  while (np > 0 && gvb_ring_offset(p.K, np) + 2 * (size_t)p.slot_bytes > (size_t)GEMV_SMEM_BUDGET) --np;
-  if (np == 0) return false;
-  const int groups = (batch + 2 * np - 1) / (2 * np), per = (batch + groups - 1) / groups;
-  np = (per + 1) / 2;
-  const size_t ring_off = gvb_ring_offset(p.K, np);
+  p.slot_bytes = gvb_slot_bytes(p.K, self.cell);
+  const size_t ring_off = gvb_ring_offset(p.K, split.np);
   const int gx = std::max(1, std::min(p.ntiles, e->num_sms));
   const int nslots = (int)std::min<size_t>(std::min(GEMV_MAX_STAGES, std::max(2, (p.ntiles + gx - 1) / gx * g.nst)), (GEMV_SMEM_BUDGET - ring_off) / p.slot_bytes);
   p.early_stages = std::max(1, std::min(nslots, (int)(gemv_early_bytes() / p.slot_bytes)));
   p.error_flag = e->d_error;
-  void (*kernel)(GemvParams, int, int, int) = np == 1 ? gemv_batch_kernel<1> : np == 2 ? gemv_batch_kernel<2> : np == 3 ? gemv_batch_kernel<3> : gemv_batch_kernel<4>;
-  launch_pdl(e->use_pdl, kernel, dim3(gx, groups), dim3(GEMV_THREADS), ring_off + (size_t)nslots * p.slot_bytes, st, p, nslots, per, batch);
+  void (*kernel)(GemvParams, int, int, int) =
+      split.np == 1 ? gemv_batch_kernel<1> : split.np == 2 ? gemv_batch_kernel<2> : split.np == 3 ? gemv_batch_kernel<3> : gemv_batch_kernel<4>;
+  launch_pdl(e->use_pdl, kernel, dim3(gx, split.groups), dim3(GEMV_THREADS), ring_off + (size_t)nslots * p.slot_bytes, st, p, nslots, split.per, batch);
   *grid = gx;
   return true;
 }
@@ -318,13 +325,13 @@ static bool launch_gemv_batch(const b200_engine* e, GemvParams p, int batch, cud
 // Fills in the launch geometry (tiles, ring slot size and depth), and starts the kernel with one
 // persistent CTA per SM (fewer when there are fewer tiles), as a programmatic dependent launch
 // when the engine allows it. Returns the grid width.
-static int launch_gemv(const b200_engine* e, GemvParams p, int batch, cudaStream_t st) {
+static int launch_gemv(const b200_engine* e, GemvParams p, int batch, cudaStream_t st, const GvbPlace* place = nullptr) {
   if (p.K % 256) throw std::runtime_error("gemv: K must be a multiple of 256");
   const GemvGeom g0 = gemv_geometry(p.seg[0].type, p.K);
   p.nblk = g0.nblk; p.nslab = g0.nslab; p.S = g0.S; p.S_last = g0.S_last; p.R = g0.R;
   if (p.epi == EPI_SWIGLU && p.nseg != 1) throw std::runtime_error("gemv: SwiGLU takes the combined gate+up image");
   int grid = 0;
-  if (launch_gemv_batch(e, p, batch, st, &grid)) return grid;
+  if (launch_gemv_batch(e, p, batch, st, place, &grid)) return grid;
   p.ntiles = 0;
   uint32_t slot = 0;
   for (int s = 0; s < p.nseg; ++s) {
@@ -512,9 +519,9 @@ struct WantedRow {
 // large batches on a single GPU, fp16 conversion (+RMSNorm) followed by the tensor-core matmul.
 // Returns the number of launches; *grid_out = partial-argmax parts per sequence (lm_head only).
 static int launch_linear(b200_engine* e, GemvParams p, int batch, cudaStream_t st, bool use_tc, int* grid_out = nullptr,
-                         void* x16_buf = nullptr) {
+                         void* x16_buf = nullptr, const GvbPlace* place = nullptr) {
   if (!use_tc) {
-    const int g = launch_gemv(e, p, batch, st);
+    const int g = launch_gemv(e, p, batch, st, place);
     if (grid_out) *grid_out = g;
     return 1;
   }
@@ -584,15 +591,21 @@ static int packed_forward_step(b200_engine* e, int batch, int nsplit, cudaStream
   }
   for (int l = 0; l < e->L; ++l) {
     const LayerW& w = e->layers[l];
+    const GemvSeg qkv[3] = {seg_of(w.wq), seg_of(w.wk), seg_of(w.wv)}, so = seg_of(w.wo), gu = seg_of(w.wgu), down = seg_of(w.wdown);
+    const GvbLaunch layer[4] = {gvb_launch(H, qkv, 3), gvb_launch(e->Hq, &so, 1), gvb_launch(H, &gu, 1), gvb_launch(F, &down, 1)};
+    auto linear = [&](const GemvParams& p, int i) {
+      const GvbPlace place{layer, 4, i};
+      return launch_linear(e, p, batch, st, use_tc, nullptr, nullptr, &place);
+    };
     {
       GemvParams p{};
-      p.seg[0] = seg_of(w.wq); p.seg[1] = seg_of(w.wk); p.seg[2] = seg_of(w.wv); p.nseg = 3;
+      p.seg[0] = qkv[0]; p.seg[1] = qkv[1]; p.seg[2] = qkv[2]; p.nseg = 3;
       p.K = H; p.x = e->d_h; p.x_stride = H; p.norm_w = w.attn_norm.f32(); p.eps = eps; p.epi = EPI_QKV_ROPE;
       if (peer) as_consumer(p);
       p.y = e->d_q; p.y_stride = e->Hq; p.y2 = e->d_kvnew; p.y2_stride = 2 * KVD;
       p.rope = e->rope; p.positions = e->d_positions; p.head_dim = e->hd; p.max_pos = e->desc.max_position_embeddings;
       p.trace = trace_rec(e, launches);
-      launches += launch_linear(e, p, batch, st, use_tc);
+      launches += linear(p, 0);
     }
     auto fill_attn = [&](AttnParams& a, int ns) {
       a.q = e->d_q; a.kv_new = e->d_kvnew; a.q_stride = e->Hq; a.kvn_stride = 2 * KVD;
@@ -626,31 +639,31 @@ static int packed_forward_step(b200_engine* e, int batch, int nsplit, cudaStream
     }
     {
       GemvParams p{};
-      p.seg[0] = seg_of(w.wo); p.nseg = 1; p.K = e->Hq; p.x = e->d_attn; p.x_stride = e->Hq; p.epi = tp ? EPI_STORE : EPI_RESID;
+      p.seg[0] = so; p.nseg = 1; p.K = e->Hq; p.x = e->d_attn; p.x_stride = e->Hq; p.epi = tp ? EPI_STORE : EPI_RESID;
       p.y = tp ? e->d_partial : e->d_h; p.y_stride = H;
       if (peer) as_producer(p, 2 * l);
       p.trace = trace_rec(e, launches);
-      launches += launch_linear(e, p, batch, st, use_tc);
+      launches += linear(p, 1);
       if (tp && !peer) launches += tp_reduce_add(e, batch, st);
     }
     {
       GemvParams p{};
-      p.seg[0] = seg_of(w.wgu); p.nseg = 1;
+      p.seg[0] = gu; p.nseg = 1;
       p.K = H; p.x = e->d_h; p.x_stride = H; p.norm_w = w.ffn_norm.f32(); p.eps = eps; p.epi = EPI_SWIGLU;
       if (peer) as_consumer(p);
       p.y = e->d_act; p.y_stride = F;
       if (use_tc) p.y16 = e->d_act;
       p.trace = trace_rec(e, launches);
-      launches += launch_linear(e, p, batch, st, use_tc);
+      launches += linear(p, 2);
     }
     {
       GemvParams p{};
-      p.seg[0] = seg_of(w.wdown); p.nseg = 1; p.K = F; p.x = e->d_act; p.x_stride = F; p.epi = tp ? EPI_STORE : EPI_RESID;
+      p.seg[0] = down; p.nseg = 1; p.K = F; p.x = e->d_act; p.x_stride = F; p.epi = tp ? EPI_STORE : EPI_RESID;
       if (use_tc) p.x16 = e->d_act;
       p.y = tp ? e->d_partial : e->d_h; p.y_stride = H;
       if (peer) as_producer(p, 2 * l + 1);
       p.trace = trace_rec(e, launches);
-      launches += launch_linear(e, p, batch, st, use_tc);
+      launches += linear(p, 3);
       if (tp && !peer) launches += tp_reduce_add(e, batch, st);
     }
   }

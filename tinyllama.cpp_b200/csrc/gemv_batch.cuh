@@ -15,8 +15,10 @@
 // Layout: the digit planes of all vectors of the CTA lie in shared memory (13.8 KB a vector at K = 4096, 37 KB at 11008) and
 // B fragments are read from there for each cell, not kept in registers. To leave room for a ring, a stage holds at most eight
 // cells; the two halves of the sixteen consumer warps take alternate stages. The host gives a CTA as many vectors as
-// leave two stages (launch_gemv); more go to further CTAs (blockIdx.y), which meet the weights in L2.
+// leave two stages (gvb_split); more go to further CTAs (blockIdx.y), which meet the weights in L2.
 #pragma once
+#include <algorithm>
+
 #include "gemv.cuh"
 
 namespace b200 {
@@ -58,6 +60,52 @@ __device__ __forceinline__ ActImage gvb_image(uint8_t* smem, int K, int np, int 
   a.xs16d = p;
   a.n16 = K / 16 + 16;
   return a;
+}
+
+// A launch as the choice between this kernel and one launch column per vector (gemv_kernel) sees it: its row length, the tiles
+// of one column and the largest cell.
+struct GvbLaunch {
+  int K, tiles, cell;
+};
+// How `batch` vectors are shared out: `per` to a CTA, np pairs of them, in `groups` groups; np = 0: a CTA has no room for two vectors
+// and two ring slots (rows beyond about 22000 elements).
+struct GvbSplit {
+  int np, groups, per;
+};
+inline uint32_t gvb_slot_bytes(int K, int cell) {
+  const GvbGeom g = gvb_geometry(K / 256);
+  return (uint32_t)((g.R * g.S * cell + 127) / 128 * 128);
+}
+inline GvbSplit gvb_split(const GvbLaunch& l, int batch) {
+  GvbSplit r{std::min(GVB_MAX, batch + 1) / 2, 0, 0};
+  while (r.np > 0 && gvb_ring_offset(l.K, r.np) + 2 * (size_t)gvb_slot_bytes(l.K, l.cell) > (size_t)GEMV_SMEM_BUDGET) --r.np;
+  if (r.np == 0) return r;
+  r.groups = (batch + 2 * r.np - 1) / (2 * r.np);
+  r.per = (batch + r.groups - 1) / r.groups;
+  r.np = (r.per + 1) / 2;
+  return r;
+}
+
+// Does launch i of n that follow one another (a layer's four, or the lm_head alone) run here? Where one column per vector finds an SM
+// for every tile at once, the columns cost what one vector costs, while this kernel's prologue grows with the vectors of a CTA. Chains of
+// one launch, us, columns / this kernel, K = 256 to 2048: 2 vectors 4.0 / 4.1, 3: 4.0 / 4.8, 4: 4.0 / 5.4, 6: 4.0 / 6.9, 8: 4.1 / 8.4
+// (K = 4096: 4.5 / 11.1); with two waves of columns 7.8 / 4.6, 5.1, 5.7, 7.1, 8.4. So:
+//   * columns for all launches where all of them fit at once, or in two waves when a CTA would take seven or eight vectors (a step of
+//     15 sequences of a 512-wide model: 83.9 us, 96.5 when its launches of 1.2 waves run here);
+//   * otherwise launch by launch, columns where they fit at once;
+//   * but not for two vectors: what the columns save there (0.1 to 0.5 us) is less than what the step loses by changing
+//     between two kernels (a layer of a 2048-wide model whose O projection alone fits: 40.0 us in columns, 38.9 here; Q8_0 41.1
+//     and 39.3; a 1024-wide one, QKV, O and down fitting: 32.0 and 30.5).
+inline bool gvb_takes(const GvbLaunch* l, int n, int i, int batch, int sms) {
+  if (batch < 2 || gvb_split(l[i], batch).np == 0) return false;
+  auto waves_fit = [&](const GvbLaunch& x, int waves) { return (long long)x.tiles * batch <= (long long)waves * sms; };
+  bool all = true;
+  for (int j = 0; j < n; ++j) {
+    const GvbSplit s = gvb_split(l[j], batch);
+    all = all && (s.np == 0 || waves_fit(l[j], s.per >= 7 ? 2 : 1));
+  }
+  if (all) return false;
+  return batch == 2 || !waves_fit(l[i], 1);
 }
 
 struct GvbShared {

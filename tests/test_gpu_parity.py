@@ -12,6 +12,7 @@ import numpy as np
 import pytest
 
 import oracle_lib as ol
+from test_host_logic import layer_launches
 
 pytestmark = pytest.mark.gpu
 GOLD = os.path.join(os.path.dirname(__file__), "golden")
@@ -127,6 +128,98 @@ def test_matvec_batches(pkg, name, rows, cols, batch):
     y = pkg.api.matvec(typ, blocks, rows, cols, x)
     for b in range(batch):
         assert rel_err(y[b], ol.matvec_f32("oracle", wd, x[b])) <= 1e-3
+
+
+@pytest.mark.parametrize("name,rows,cols,batch,per", [("q4_k", 40000, 256, 2, 2), ("q6_k", 20010, 512, 3, 3), ("q6_k", 5000, 768, 8, 8), ("q8_0", 9000, 1024, 5, 5),
+                                                      ("q8_0", 12000, 1280, 6, 6), ("q4_k", 9000, 2048, 15, 8), ("q4_k", 3000, 14336, 7, 2), ("q4_k", 2400, 22016, 3, 2)])
+def test_matvec_of_several_vectors(pkg, name, rows, cols, batch, per):
+    """As above, with the kernel named: every case runs on the several-vector kernel with `per` vectors to a CTA. One to four pairs
+    of vectors, several row groups per tile (eight, four, two) with a last tile that is not full, one and several groups of
+    vectors, rows that leave room for a single pair. Tolerance: that of the matvec."""
+    typ = TYPES[name]
+    assert pkg.api.matvec_plan([(cols, [(typ, rows)])], batch) == [per]
+    blocks = pkg.synth.quantize(typ, pkg.synth.fill_normal(rows * cols, 95, rows + typ, 0.02))
+    wd = ol.dequant("oracle", typ, blocks).reshape(rows, cols)
+    x = pkg.synth.fill_normal(batch * cols, 96, cols, 1.0).reshape(batch, cols)
+    y = pkg.api.matvec(typ, blocks, rows, cols, x)
+    for b in range(batch):
+        assert rel_err(y[b], ol.matvec_f32("oracle", wd, x[b])) <= 1e-3
+
+
+# Two layers of models wide enough for the several-vector kernel; the second has two row groups to a tile and rows of eleven blocks.
+WIDE = {"w2048": (dict(hidden=2048, ffn=5632, n_heads=32, n_kv_heads=4, n_layers=2, vocab=8192, max_pos=64, theta=10000.0), 1),
+        "w1024": (dict(hidden=1024, ffn=2816, n_heads=16, n_kv_heads=4, n_layers=2, vocab=8192, max_pos=64, theta=10000.0), 0)}
+
+
+@pytest.fixture(scope="module")
+def wide(pkg, tmp_path_factory):
+    """name -> (model file, 15 ragged prompts, tokens of two steps, the oracle's logits of those steps [2][15][vocab])."""
+    made = {}
+
+    def get(name):
+        if name not in made:
+            shape, scheme = WIDE[name]
+            path = pkg.synth.write_gguf(str(tmp_path_factory.mktemp("wide") / f"{name}.gguf"), shape, scheme=scheme, norm_random=True)
+            rng = np.random.default_rng(41)
+            prompts = [rng.integers(0, shape["vocab"], 1 + 3 * b % 4) for b in range(15)]
+            toks = rng.integers(0, shape["vocab"], (2, 15))
+            orc = ol.OracleModel.from_gguf(path, max_seqs=15)
+            refs = np.empty((2, 15, shape["vocab"]), np.float32)
+            for b, ids in enumerate(prompts):
+                for pos, t in enumerate(ids):
+                    orc.decode(int(t), pos, seq=b)
+                for k in range(2):
+                    refs[k, b] = orc.decode(int(toks[k, b]), len(ids) + k, seq=b)
+            made[name] = path, prompts, toks, refs
+        return made[name]
+
+    return get
+
+
+@pytest.mark.parametrize("batch", [2, 3, 5, 9, 15])
+@pytest.mark.parametrize("name", list(WIDE))
+def test_steps_of_several_sequences_on_wide_models(pkg, wide, name, batch):
+    """Steps of 2 to 15 sequences whose launches share their weights: RMSNorm prologue, q/k/v of mixed block types with RoPE at ragged
+    positions, residual, SwiGLU, logits and their first maxima, shuffled KV slots. Tolerance: the 24-bit activations' (1e-4 on
+    logits of about 1, as for the toy models)."""
+    shape, scheme = WIDE[name]
+    qo, v, gu, down = (12, 14, 12, 14) if scheme == 1 else (8, 8, 8, 8)
+    plan = pkg.api.matvec_plan(layer_launches(shape, qo, v, gu, down), batch) + pkg.api.matvec_plan([(shape["hidden"], [(down, shape["vocab"])])], batch)
+    assert all(plan) if name == "w2048" or batch == 2 else plan[2] and plan[4]
+    path, prompts, toks, refs = wide(name)
+    eng = pkg.Engine.from_gguf(path, max_seqs=16)
+    slots = [int(s) for s in np.random.default_rng(batch).permutation(16)[:batch]]
+    for b in range(batch):
+        eng.prefill(prompts[b], slot=slots[b])
+    for k in range(2):
+        logits, amax = eng.decode(toks[k, :batch], [len(prompts[b]) + k for b in range(batch)], slots=slots)
+        assert np.array_equal(amax, logits.argmax(axis=1))
+        worst = float(np.abs(logits - refs[k, :batch]).max())
+        assert worst <= 1e-4, worst
+    eng.close()
+
+
+@pytest.mark.parametrize("penalty", [1.0, 1.3])
+def test_greedy_loop_of_several_sequences_on_a_wide_model(pkg, wide, penalty):
+    """The device-resident loop over the several-vector kernel (three sequences, 16 steps), with and without the repetition penalty in
+    its lm_head epilogue: every id is the first maximum of the oracle's (penalised) logits, up to near-ties of 1e-3."""
+    path = wide("w2048")[0]
+    eng = pkg.Engine.from_gguf(path, max_seqs=3)
+    orc = ol.OracleModel.from_gguf(path, max_seqs=3)
+    firsts, hist = [5, 4000, 77], [[9, 5], [4000], []]
+    if penalty == 1.0:
+        out, _ = eng.generate_greedy(firsts, [0, 0, 0], 16)
+    else:
+        out, _ = eng.generate_greedy_penalized(firsts, [0, 0, 0], 16, penalty, histories=hist)
+    eng.close()
+    for b in range(3):
+        gen, tok = list(hist[b]), firsts[b]
+        for pos in range(16):
+            lg = orc.decode(tok, pos, seq=b)
+            lg = _penalise(lg, gen, penalty) if penalty != 1.0 else lg
+            tok = int(out[pos, b])
+            assert lg[tok] >= lg.max() - 1e-3, (b, pos, tok, int(lg.argmax()))
+            gen.append(tok)
 
 
 def test_matvec_batch_and_edge_values(pkg):

@@ -546,7 +546,7 @@ def main():
 
     clocks = sampler.finish()
     if on_tc:
-        # batch >= 16: the linear layers run on the tcgen05 matmul (with its fp16 conversion and split-K reduction). Below
+        # batch >= 16: the linear layers run on the tcgen05 matmul (with its fp16 conversion). Below
         # ~128 tokens the matmul is still bound by the packed weight bytes (2 * batch / 0.5625 FLOP per byte against a
         # machine balance of ~250), so the roofline stays the HBM one; the tensor throughput is reported beside it.
         tf = ksum_f / ksum_t / 1e6

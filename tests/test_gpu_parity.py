@@ -761,3 +761,19 @@ def test_two_layer_models_of_the_large_shapes(pkg, tmp_path, shape, scheme, kv):
     tol = 1.5e-2 * float(np.abs(ref).max()) if i8 else 2e-2
     assert np.abs(got - ref).max() <= tol
     eng.close()
+
+
+def test_kernel_timing_counts_the_batch_in_the_steps_formats(pkg, tiny_models):
+    """Bytes of the timed launches of the batched path: packed weights, norm vectors and the batch's activations as the step moves
+    them, which is in fp16 from the SwiGLU to the down projection and from the prompt attention on."""
+    B, ctx = 16, 128
+    eng = pkg.Engine.from_gguf(tiny_models[1], max_seqs=B, max_ctx=ctx)
+    g = pkg.gguf.GGUF(tiny_models[1])
+    size = lambda *names: sum(g.tensors[f"blk.0.{n}.weight"]["data"].nbytes for n in names)
+    H, F, kvd = 256, 512, 128
+    want = {0: size("ffn_gate", "ffn_up") + 4 * H + B * (4 * H + 2 * F), 1: size("attn_q", "attn_k", "attn_v") + 4 * H + B * 4 * (2 * H + 2 * kvd),
+            2: size("attn_output") + B * 8 * H, 3: size("ffn_down") + B * (2 * F + 4 * H), 5: ctx * 8 * kvd + ctx * 6 * H}
+    for which, nbytes in want.items():
+        us, got = eng.time_kernel(16 + which, 4)
+        assert us > 0 and got == nbytes, (which, got, nbytes)
+    eng.close()

@@ -54,6 +54,7 @@ struct alignas(64) DgmMaps {
 
 struct DgmShared {
   unsigned long long full[DGM_MAX_STAGES], empty[DGM_MAX_STAGES], acc_full[2], acc_empty[2];
+  unsigned long long drained;  // all MMAs issued by this CTA have completed
   uint32_t tmem_base;
   int abort_flag, issued;  // issued: K slices whose copies have been requested
   int last;
@@ -161,6 +162,7 @@ __global__ void __launch_bounds__(DGM_THREADS, 1) dense_gemm_kernel(const __grid
   if (tid == 0) {
     for (int i = 0; i < DGM_MAX_STAGES; ++i) { mbar_init(&sh.full[i], 1); mbar_init(&sh.empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&sh.acc_full[i], 1); mbar_init(&sh.acc_empty[i], DGM_EPI_WARPS); }
+    mbar_init(&sh.drained, 1);
     sh.abort_flag = 0;
     sh.issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -227,6 +229,9 @@ __global__ void __launch_bounds__(DGM_THREADS, 1) dense_gemm_kernel(const __grid
       }
       if (ok) tc_commit_if(leader, &sh.acc_full[buf]);
     }
+    // the block frees the tensor memory that MMAs in flight write: the epilogue waits for them too, but not after a give-up
+    tc_commit_if(leader, &sh.drained);
+    mbar_wait(&sh.drained, 0);
     __syncwarp();
   } else {
     // ---- epilogue warps: lanes 32 (w & 3) .. of the accumulator = weight rows, the two groups of four split the tokens ----
@@ -298,7 +303,7 @@ __global__ void __launch_bounds__(DGM_THREADS, 1) dense_gemm_kernel(const __grid
   }
   tc_fence_before();
   __syncthreads();
-  // The MMA lane waits for every copy; only after a give-up may some still be in flight, and the block outlives them.
+  // The MMA warp waits for every copy; only after a give-up may some still be in flight, and the block outlives them.
   if (sh.abort_flag && tid == 0)
     for (int s = max(0, sh.issued - p.stages); s < sh.issued; ++s) mbar_wait(&sh.full[s % p.stages], (uint32_t)((s / p.stages) & 1));
   if (warp == 0) tc_dealloc(tmem, 2 * p.acc_cols);

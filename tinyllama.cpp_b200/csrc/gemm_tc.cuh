@@ -23,7 +23,7 @@
 // block, byte permutes at half rate, 1650 cycles a block and warp beside 1240 of MMA issue, where HBM would need 800. With 256
 // tokens it is the activation tiles: 128 KB a block and SM from L2, at about 36 bytes a cycle.
 // The roles meet on mbarriers only. Every wait is bounded; on a give-up the kernel sets the error word,
-// waits for its copies, frees its tensor memory and returns.
+// waits for its MMAs and copies, frees its tensor memory and returns.
 //
 // Why the A operand goes through tensor memory: with few tokens the kernel should run at the rate the
 // packed weights arrive (128 rows x 64 elements of Q4_K in about 200 cycles). Stored to shared memory, the
@@ -301,6 +301,7 @@ struct TcShared {
   unsigned long long acc_empty[2];           // the sixteen warps have read the accumulator
   unsigned long long w_full[TC_W_STAGES];    // the packed units of a block have landed
   unsigned long long w_empty[TC_W_STAGES];   // the sixteen warps have copied their part of the stage into registers
+  unsigned long long drained;                // all MMAs issued by this CTA have completed
   uint32_t tmem_base;
   int abort_flag;
   int last;       // this CTA is the last one of a cut tile
@@ -524,6 +525,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     for (int i = 0; i < TC_B_STAGES; ++i) { mbar_init(&sh.b_full[i], 1); mbar_init(&sh.b_empty[i], 1); }
     for (int i = 0; i < TC_W_STAGES; ++i) { mbar_init(&sh.w_full[i], 1); mbar_init(&sh.w_empty[i], TC_WORKERS / 32); }
     for (int i = 0; i < 2; ++i) { mbar_init(&sh.acc_full[i], 1); mbar_init(&sh.acc_empty[i], TC_WORKERS / 32); }
+    mbar_init(&sh.drained, 1);
     sh.abort_flag = 0;
     sh.w_issued = sh.b_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -578,6 +580,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
       }
       if (ok) tc_commit_if(leader, &sh.acc_full[buf]);
     }
+    // the block frees the tensor memory that MMAs in flight write: the epilogue waits for them too, but not after a give-up
+    tc_commit_if(leader, &sh.drained);
+    mbar_wait(&sh.drained, 0);
     __syncwarp();
   } else if (warp == TC_WORKERS / 32 + 2) {
     // ---- activation producer ----

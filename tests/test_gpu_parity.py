@@ -576,7 +576,8 @@ def test_prefill_batch_equals_one_call_per_sequence(pkg, tiny_models, kv):
     """Sequence-aware ingestion of ragged prompts in shared 512-token chunks (nine sequences, 860 tokens: two chunks, a
     prompt that straddles the chunk border, prompts shorter than a tile) against one b200_prefill call per sequence:
     logits and the following decode step agree to 1e-4 (each token's matmul column and attention rows are its own, so
-    the two differ at most by the order of a few fp32 additions where a prompt straddles a chunk border); and against
+    the two differ at most by the order of a few fp32 additions where a prompt straddles a chunk border; rows longer than
+    these may also be cut along K at other places when the chunk holds more tokens); and against
     the oracle with the tensor-core path's tolerance."""
     kvd = pkg.KV_I8 if kv == "i8" else pkg.KV_F32
     lens = [120, 17, 100, 127, 64, 99, 111, 125, 97]

@@ -51,6 +51,8 @@ __device__ __forceinline__ int dp4a_ss(uint32_t a, uint32_t b, int c) {
   return d;
 }
 
+__device__ __forceinline__ uint32_t u4_word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
 __device__ __forceinline__ float half_bits_to_float(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 
 __device__ __forceinline__ float warp_sum(float v) {

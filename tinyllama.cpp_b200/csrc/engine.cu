@@ -254,7 +254,7 @@ static GemvSeg seg_of(const DevTensor& t) {
   const GemvGeom g = gemv_geometry(t.type, (int)t.cols);
   GemvSeg s;
   s.img = t.base; s.type = t.type; s.rows = (int)t.img_rows; s.tiles = t.tiles;
-    s.stage_bytes = g.stage_bytes; s.stage_bytes_last = g.stage_bytes_last; s.tile_bytes = g.tile_bytes;
+  s.stage_bytes = g.stage_bytes; s.stage_bytes_last = g.stage_bytes_last; s.tile_bytes = g.tile_bytes;
   return s;
 }
 
@@ -322,9 +322,9 @@ static bool launch_gemv_batch(const b200_engine* e, GemvParams p, int batch, cud
   return true;
 }
 
-// Fills in the launch geometry (tiles, ring slot size and depth), and starts the kernel with one
-// persistent CTA per SM (fewer when there are fewer tiles), as a programmatic dependent launch
-// when the engine allows it. Returns the grid width.
+// Starts the matvec of one or several vectors as a programmatic dependent launch when the engine allows it: several on the kernel
+// that shares the weights (launch_gemv_batch), or on one launch column each, with one persistent CTA per SM and column (fewer
+// when there are fewer tiles). Fills in the geometry: tiles, ring slot size and depth. Returns the grid width.
 static int launch_gemv(const b200_engine* e, GemvParams p, int batch, cudaStream_t st, const GvbPlace* place = nullptr) {
   if (p.K % 256) throw std::runtime_error("gemv: K must be a multiple of 256");
   const GemvGeom g0 = gemv_geometry(p.seg[0].type, p.K);
@@ -349,21 +349,9 @@ static int launch_gemv(const b200_engine* e, GemvParams p, int batch, cudaStream
   p.early_stages = std::max(1, std::min(nstages, (int)(gemv_early_bytes() / p.slot_bytes)));
   p.error_flag = e->d_error;
   const size_t smem = ring_off + (size_t)nstages * p.slot_bytes;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(gx, batch);
-  cfg.blockDim = dim3(GEMV_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = e->use_pdl ? 1 : 0;
-  if (e->P == 2) CK(cudaLaunchKernelEx(&cfg, gemv_kernel<2>, p, nstages));
-  else CK(cudaLaunchKernelEx(&cfg, gemv_kernel<3>, p, nstages));
+  launch_pdl(e->use_pdl, e->P == 2 ? gemv_kernel<2> : gemv_kernel<3>, dim3(gx, batch), dim3(GEMV_THREADS), smem, st, p, nstages);
   return gx;
 }
-
 
 // Starts the tensor-core matmul for T tokens (gemm_tc.cuh). x16: [T][K] fp16 activations.
 static void encode_map(CUtensorMap* tm, CUtensorMapDataType dt, int rank, const void* base, const cuuint64_t* gdim, const cuuint64_t* gstr,
@@ -515,8 +503,8 @@ struct WantedRow {
 
 #include "block_engine.inc"
 
-// One fused linear layer of the step: the matvec kernel (one launch column per sequence), or, for
-// large batches on a single GPU, fp16 conversion (+RMSNorm) followed by the tensor-core matmul.
+// One fused linear layer of the step: a matvec kernel (launch_gemv; place as there), or, for large batches and prompt chunks, fp16
+// conversion (+RMSNorm; none where p.x16 is given) followed by the tensor-core matmul.
 // Returns the number of launches; *grid_out = partial-argmax parts per sequence (lm_head only).
 static int launch_linear(b200_engine* e, GemvParams p, int batch, cudaStream_t st, bool use_tc, int* grid_out = nullptr,
                          void* x16_buf = nullptr, const GvbPlace* place = nullptr) {

@@ -191,8 +191,6 @@ __device__ __forceinline__ void tc_affine4(uint32_t bytes, uint64_t D, uint64_t 
   w1 = f2_half2(f2_fma(f2_pack(byte_to_unit_float(bytes, 2), byte_to_unit_float(bytes, 3)), D, C));
 }
 
-__device__ __forceinline__ uint32_t u4_word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
-
 // The packed bytes one thread needs for its 64 elements [64 c, 64 c + 64) of a block, copied from the ring so that
 // the stage can be refilled while they are converted. cell, r: the row's cell and its row in it.
 //   Q4_K: r[0] = d, dmin, 12 scale bytes; r[1..2] = 32 nibble pairs (low nibbles = elements 0..31, high = 32..63)

@@ -10,7 +10,8 @@
 // 85 % of the issue slots at the rate HBM delivers the cell; one launch column per vector therefore took 5 x the time for 5
 // vectors (62 us a launch for 5 sequences of a 7B Q4_K model, 14 us for one). A further pair costs about 110 instructions
 // here (Q6_K: 180): 28 to 45 us a launch, 6.9 -> 4.4 ms for that model's step of 5 sequences over 600 tokens. (The integer
-// MMA itself is not the limit: 8.1 cycles per SM quarter.)
+// MMA itself is not the limit: 8.1 cycles per SM quarter.) At the 96 registers that 17 warps leave a
+// thread, four pairs spill 176 bytes, three 76, two 16.
 //
 // Layout: the digit planes of all vectors of the CTA lie in shared memory (13.8 KB a vector at K = 4096, 37 KB at 11008) and
 // B fragments are read from there for each cell, not kept in registers. To leave room for a ring, a stage holds at most eight
@@ -94,8 +95,8 @@ inline GvbSplit gvb_split(const GvbLaunch& l, int batch) {
 //     15 sequences of a 512-wide model: 83.9 us, 96.5 when its launches of 1.2 waves run here);
 //   * otherwise launch by launch, columns where they fit at once;
 //   * but not for two vectors: what the columns save there (0.1 to 0.5 us) is less than what the step loses by changing
-//     between two kernels (a layer of a 2048-wide model whose O projection alone fits: 40.0 us in columns, 38.9 here; Q8_0 41.1
-//     and 39.3; a 1024-wide one, QKV, O and down fitting: 32.0 and 30.5).
+//     between two kernels (steps of 8 layers, launch by launch / here: 2048 wide, where the O projection alone fits, 320.8 / 311.8
+//     us, in Q8_0 329.7 / 315.9; 1024 wide, where QKV, O and down fit, 256.5 / 245).
 inline bool gvb_takes(const GvbLaunch* l, int n, int i, int batch, int sms) {
   if (batch < 2 || gvb_split(l[i], batch).np == 0) return false;
   auto waves_fit = [&](const GvbLaunch& x, int waves) { return (long long)x.tiles * batch <= (long long)waves * sms; };
@@ -140,8 +141,6 @@ struct GvbLane {
 };
 
 // ph, pq as in compute_q4 / q6 / q8: one cell times all vectors; acc[v][0 / 1] = rows g / g + 8.
-__device__ __forceinline__ uint32_t u4_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
-
 template <int NP>
 __device__ __forceinline__ void gvb_q4(const uint8_t* ph, const uint8_t* pq, uint8_t* smem, int K, int blk, const GvbLane& G, float (&acc)[2 * NP][2]) {
   const LaneCtx& L = G.L;
@@ -212,7 +211,7 @@ __device__ __forceinline__ void gvb_q6(const uint8_t* ph, const uint8_t* pq, uin
           return nib | (top & 0x30303030u);
         };
         const uint32_t a0 = six(la.x, ha.x), a1 = six(lb.x, hb.x), a2 = six(la.y, ha.y), a3 = six(lb.y, hb.y);
-        const uint32_t w0 = u4_of(sc0, 2 * h + hi), w1 = u4_of(sc1, 2 * h + hi);
+        const uint32_t w0 = u4_word(sc0, 2 * h + hi), w1 = u4_word(sc1, 2 * h + hi);
         const int k00 = byte_s(w0, 2 * q), k01 = byte_s(w0, 2 * q + 1), k10 = byte_s(w1, 2 * q), k11 = byte_s(w1, 2 * q + 1);
 #pragma unroll
         for (int v = 0; v < 2 * NP; ++v) {
@@ -248,8 +247,8 @@ __device__ __forceinline__ void gvb_q8(const uint8_t* ph, const uint8_t* pq, uin
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const uint2 qa = *reinterpret_cast<const uint2*>(pq + 512 * j), qb = *reinterpret_cast<const uint2*>(pq + 512 * j + 128);
-    const float d0 = scale_field_to_float((uint16_t)((u4_of(da, j >> 1) >> (16 * (j & 1))) & 0xFFFF));
-    const float d1 = scale_field_to_float((uint16_t)((u4_of(db, j >> 1) >> (16 * (j & 1))) & 0xFFFF));
+    const float d0 = scale_field_to_float((uint16_t)((u4_word(da, j >> 1) >> (16 * (j & 1))) & 0xFFFF));
+    const float d1 = scale_field_to_float((uint16_t)((u4_word(db, j >> 1) >> (16 * (j & 1))) & 0xFFFF));
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
       const uint2 b = *reinterpret_cast<const uint2*>(bp + i * G.pair_step + 32 * j);

@@ -522,16 +522,13 @@ def main():
         ksum_t += us * per_step
         ksum_f += flops * per_step
     gemv_launches = sum(v[1] for v in kinds.values())
-    # DRAM bytes (read + write) per launch from one ncu capture of this workload's four per-layer kinds
-    # (profiles/gemv_kernel_7b_q4km_bs1.txt); the lm_head launch was not captured and is scaled from its
-    # algorithmic bytes by the mean ratio of the others. Other workloads: no capture, null.
+    # DRAM bytes (read + write) per launch from one ncu capture of this workload's kinds
+    # (profiles/gemv_kernel_7b_q4km_bs1.txt). Other workloads: no capture, null.
     traffic = traffic_source = None
     if args.workload == "c3-llama2-7b-q4km-bs1" and world == 1:
         traffic_source = "profiles/gemv_kernel_7b_q4km_bs1.txt (one ncu capture of the same launches; not measured in this run)"
-        ncu_mb = {"gate_up_swiglu": 51.530, "qkv_rope": 32.998, "down_proj": 38.268, "o_proj": 9.667}
-        ratio = sum(ncu_mb.values()) * 1e6 / sum(kern[k]["bytes"] for k in ncu_mb)
-        tot = sum(ncu_mb[k] * 1e6 * kinds[k][1] for k in ncu_mb) + ratio * kern["lm_head"]["bytes"]
-        traffic = int(tot / gemv_launches)
+        ncu_mb = {"gate_up_swiglu": 50.826, "qkv_rope": 32.752, "down_proj": 37.124, "o_proj": 9.539, "lm_head": 109.141}
+        traffic = int(sum(ncu_mb[k] * 1e6 * kinds[k][1] for k in ncu_mb) / gemv_launches)
     achieved = ksum_b / ksum_t / 1e3  # GB/s
     ctx_sum_mid = sum(lens) + batch * (warmup + args.steps / 2.0)  # context positions read per step, over all sequences, mid-run
     # per-rank shares add up to the whole model over the ranks (norm vectors are replicated: negligible)

@@ -331,6 +331,25 @@ def test_attention_decode(pkg, kv_i8, nq, nkv, hd, n_ctx, splits):
     assert np.abs(out - ref).max() <= 2e-5 * max(1.0, np.abs(ref).max())
 
 
+# A tile of the cluster kernel holds 4096 bytes of keys: 32 / 64 INT8 or 8 / 16 FP32 rows of 128 / 64 elements; the 4 warps of each of
+# 1, 2, 4 or 8 splits take tiles in turn through a ring of two. Contexts: nothing cached, tile edges and remainders, rings that wrap,
+# more warps than tiles, the new row in every place of the sequence of warps.
+@pytest.mark.parametrize("kv_i8", [False, True])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+def test_attention_decode_clusters(pkg, kv_i8, hd, splits):
+    rows = 4096 // (hd * (1 if kv_i8 else 4))
+    nq, nkv = (6, 2) if splits < 4 else (3, 3)
+    for n_ctx in (0, 1, rows - 1, rows, rows + 1, 3 * rows + 5, 4 * splits * rows, 4 * splits * rows + 1, 9 * splits * rows + rows // 2 + 1):
+        rng = np.random.default_rng(n_ctx + hd + splits)
+        q = rng.standard_normal(nq * hd).astype(np.float32)
+        kc = rng.standard_normal((n_ctx + 1, nkv, hd)).astype(np.float32)
+        vc = rng.standard_normal((n_ctx + 1, nkv, hd)).astype(np.float32)
+        ref = ol.attention_decode(q, kc, vc, nq, nkv, hd, kv_int8=kv_i8)
+        out = pkg.api.attention_decode(q, kc[-1], vc[-1], kc[:-1], vc[:-1], nq, nkv, hd, kv_dtype=pkg.KV_I8 if kv_i8 else pkg.KV_F32, n_splits=splits)
+        assert np.abs(out - ref).max() <= 2e-5 * max(1.0, np.abs(ref).max()), n_ctx
+
+
 @pytest.mark.parametrize("kv_i8", [False, True])
 @pytest.mark.parametrize("nq,nkv,hd,n_ctx,n_tok", [(4, 2, 64, 40, 40), (4, 4, 64, 130, 1), (8, 2, 128, 333, 77),
                                                   (32, 8, 128, 1100, 256), (2, 1, 128, 64, 64), (2, 2, 64, 65, 65)])

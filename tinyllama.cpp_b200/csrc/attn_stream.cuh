@@ -1,0 +1,430 @@
+// Decode attention of one new token per sequence (head sizes 64 and 128): one thread-block cluster per (query head, sequence), whose
+// warps share out the context and meet once, through distributed shared memory.
+//
+// What bounds it: latency. A layer of a 7B model holds 8 MB of INT8 keys and values at 1000 positions, 1.3 us of HBM time; the rest is a
+// chain of dependent steps between the QKV launch's last store and the O projection's first load, with one warp per scheduler. So:
+//   * cached rows do not depend on the launch before: every warp requests its first two tiles (bulk copies into its own ring) before it
+//     waits for that launch, and more as it goes;
+//   * a warp works alone: tiles of 4096 bytes of keys and as much of values, an online softmax over its own rows, scores that never
+//     leave registers, no branch between the loads of a tile (with one per load a tile took 2 us);
+//   * INT8 scores on the integer tensor cores, q as 24-bit digit planes as the matvec's activations (gemv.cuh): 8 MMAs for a tile where
+//     conversions and FMAs took 320 instructions. INT8 values become FP32 through a byte permute and one exact subtraction of a pair
+//     (I2F runs at a sixteenth of the FMA rate);
+//   * one cluster barrier: each warp stores its output, cut by dimensions, into the blocks that finish those dimensions. (Partials through
+//     global memory, a ticket and a merge by the last block: attn_decode_kernel, 5 us a launch.)
+// The warp that would have the next tile appends the new row (quantised when the cache is INT8) and attends to it from registers.
+// Measured, us from the QKV launch's end to the output: 7B INT8, 1030 positions 6.9 (and 11.2 until the O projection's end) before,
+// 7.7 (6.0) with 4 splits; 1.1B FP32, 150 positions 4.3 (8.2) and 3.4 (4.3); the O projection no longer queues behind 608 blocks.
+// Whole steps: 7B 1.82 -> 1.67 ms, 5 sequences 4.39 -> 4.18, 16 sequences 4.70 -> 3.99; 1.1B greedy, 25 steps 17.5 -> 15.1 ms.
+//
+// Arithmetic as in attn.cuh (reference model.cpp:632-663, utils.cpp:675-698; INT8 quantizer cuda_kernels.cu:1535-1549, 1596-1599), the
+// softmax in its online form: o = sum_t 2^(s_t - M) v_t / (sum_t 2^(s_t - M) + 1e-9), s_t = (q . k_t) log2(e) / sqrt(hd).
+#pragma once
+#include "attn.cuh"
+#include "gemv.cuh"
+
+namespace b200 {
+
+constexpr int ATS_WARPS = 4, ATS_THREADS = 32 * ATS_WARPS;
+constexpr int ATS_MAX_CLUSTER = 8;
+constexpr int ATS_PASSES = 8;           // 512-byte pieces of a tile: one 16-byte load per lane each
+constexpr int ATS_TILE = ATS_PASSES * 512;
+constexpr int ATS_DEPTH = 2;            // tiles in flight per warp
+
+__host__ __device__ __forceinline__ size_t ats_smem_bytes() { return (size_t)ATS_WARPS * ATS_DEPTH * 2 * ATS_TILE; }
+
+__device__ __forceinline__ uint32_t cluster_map(uint32_t smem, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// four signed bytes as two exact FP32 pairs: 0x4B0000uu is 8388608 + u, u = byte + 128
+__device__ __forceinline__ void ats_cvt4(uint32_t w, uint64_t& a, uint64_t& b) {
+  w ^= 0x80808080u;
+  const uint64_t off = f2_dup(-8388736.0f);
+  a = f2_add(f2_pack(__byte_perm(w, 0x4B000000u, 0x7440), __byte_perm(w, 0x4B000000u, 0x7441)), off);
+  b = f2_add(f2_pack(__byte_perm(w, 0x4B000000u, 0x7442), __byte_perm(w, 0x4B000000u, 0x7443)), off);
+}
+
+// c += A(16x32, s8) * B(32x8, s8)
+__device__ __forceinline__ void imma_acc(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <bool KV_I8, int HD>
+__global__ void __launch_bounds__(ATS_THREADS, 20 / ATS_WARPS) attn_stream_kernel(const AttnParams prm) {
+  constexpr int EPL = KV_I8 ? 16 : 4;           // elements of a 16-byte piece
+  constexpr int ROWB = HD * (KV_I8 ? 1 : 4);    // bytes of a row
+  constexpr int LPP = ROWB / 16, RPP = 32 / LPP;  // lanes per row, rows per pass
+  constexpr int ROWS = ATS_PASSES * RPP;        // rows per tile
+  constexpr int NS = LPP < ATS_PASSES ? ATS_PASSES / LPP : 1;  // rows of a tile whose scores a lane ends up with
+  constexpr int DUP = LPP > ATS_PASSES ? LPP / ATS_PASSES : 1; // lanes that hold the same row's score
+  constexpr int NP2 = EPL / 2;                  // FP32 pairs of a piece
+  constexpr int DPL = HD / 32;                  // output dimensions a lane ends up with
+  extern __shared__ __align__(128) uint8_t ats_smem[];
+  __shared__ unsigned long long full[ATS_WARPS][ATS_DEPTH];
+  __shared__ __align__(16) float vn_s[HD];
+  __shared__ __align__(16) uint8_t q_s[KV_I8 ? ATS_WARPS : 1][3][HD];
+  __shared__ __align__(16) float part[ATS_WARPS * HD];  // [warps of the cluster][HD / cluster]
+  __shared__ __align__(16) float2 ml[ATS_WARPS * ATS_MAX_CLUSTER];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int C = gridDim.x, split = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int G = prm.nq / prm.nkv, kvh = h / G;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  unsigned long long* rec = (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) ? prm.trace : nullptr;
+  trace_stamp(rec, 0);
+  if (C > 1) cluster_arrive();  // every block of the cluster has started before any stores into another's memory
+
+  // positions and slots are set between steps, cached rows by earlier steps: neither waits for the launch before this one
+  const int pos = prm.positions[b], slot = prm.slots[b];
+  const bool bad = pos < 0 || pos >= prm.max_ctx;  // would lie outside the caller's buffers
+  const int cached = bad ? 0 : prm.cached_new ? pos + 1 : pos;  // rows that come from the cache
+  const int ntiles = (cached + ROWS - 1) / ROWS, nw = ATS_WARPS * C, gw = split * ATS_WARPS + warp;
+  const size_t crow0 = ((size_t)slot * prm.nkv + kvh) * prm.max_ctx;  // row of position 0
+  uint8_t* ring = ats_smem + (size_t)warp * ATS_DEPTH * 2 * ATS_TILE;
+  if (lane == 0) {
+    for (int i = 0; i < ATS_DEPTH; ++i) mbar_init(&full[warp][i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  auto request = [&](int tile, int s) {  // lane 0
+    const int r0 = tile * ROWS;
+    const uint32_t bytes = (uint32_t)min(ROWS, cached - r0) * ROWB;
+    const size_t at = (crow0 + r0) * ROWB;
+    mbar_expect_tx(&full[warp][s], 2 * bytes);
+    bulk_g2s(ring + (size_t)s * 2 * ATS_TILE, static_cast<const uint8_t*>(prm.k_cache) + at, bytes, &full[warp][s]);
+    bulk_g2s(ring + (size_t)s * 2 * ATS_TILE + ATS_TILE, static_cast<const uint8_t*>(prm.v_cache) + at, bytes, &full[warp][s]);
+  };
+  if (lane == 0)
+    for (int i = 0; i < ATS_DEPTH; ++i)
+      if (gw + i * nw < ntiles) request(gw + i * nw, i);
+  const int gl = lane % LPP, gi = lane / LPP;
+  // the i-th row of a tile whose score this lane ends up with (see the two ways of the scores)
+  auto row_of = [&](int i) { return KV_I8 ? 8 * (NS * (lane & 3) + i) + (lane >> 2) : gl / DUP * RPP + gi; };
+  float ksc[NS], vsc[NS];  // scales of the next tile's rows
+  auto scales = [&](int tile) {
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      const int t = tile * ROWS + row_of(i);
+      ksc[i] = vsc[i] = 1.f;
+      if (KV_I8 && t < cached) { ksc[i] = __ldcg(prm.k_scale + crow0 + t); vsc[i] = __ldcg(prm.v_scale + crow0 + t); }
+    }
+  };
+  scales(gw);
+  __syncwarp();
+
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // q, the new rows and the output belong to the launch before until here
+  for (int i = 1; i < 5; ++i) trace_stamp(rec, i);
+  if (bad) {  // nothing read, nothing appended
+    if (split == 0 && tid < HD) prm.out[(size_t)b * prm.out_stride + h * HD + tid] = __int_as_float(0x7fc00000);
+    if (tid == 0 && prm.error_flag) *reinterpret_cast<volatile int*>(prm.error_flag) = 3;
+    if (C > 1) cluster_wait();
+    return;
+  }
+  const float* qg = prm.q + (size_t)b * prm.q_stride + h * HD;
+  uint64_t q[2] = {0ull, 0ull};  // FP32 cache: this lane's four elements
+  uint4 qf[KV_I8 ? HD / 64 : 1];  // INT8 cache: 24-bit digit planes of q as the integer MMA's B operand (column 2 p: plane p)
+  float qscale = 1.f;
+  if (KV_I8) {
+    float v[DPL], amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) {
+      v[i] = qg[lane * DPL + i];
+      amax = fmaxf(amax, fabsf(v[i]));
+    }
+    amax = warp_max(amax);
+    constexpr int QMAX = 8355711;  // largest magnitude of three balanced base-256 digits
+    qscale = amax * (1.0f / (float)QMAX);
+    const float inv = amax > 0.f ? __fdividef((float)QMAX, amax) : 0.f;
+    uint32_t u[DPL];
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) u[i] = (uint32_t)(max(-QMAX, min(QMAX, __float2int_rn(v[i] * inv))) + 0x808080);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      uint32_t w = 0;
+#pragma unroll
+      for (int i = 0; i < DPL; ++i) w |= (((u[i] >> (8 * p)) & 0xFFu) ^ 0x80u) << (8 * i);
+      if (DPL == 4) *reinterpret_cast<uint32_t*>(&q_s[warp][p][lane * 4]) = w;
+      else *reinterpret_cast<uint16_t*>(&q_s[warp][p][lane * 2]) = (uint16_t)w;
+    }
+    __syncwarp();
+    const int col = lane >> 2;
+#pragma unroll
+    for (int j = 0; j < HD / 64; ++j)
+      qf[j] = (col & 1) || col > 4 ? make_uint4(0u, 0u, 0u, 0u) : *reinterpret_cast<const uint4*>(&q_s[warp][col >> 1][64 * j + 16 * (lane & 3)]);
+  } else {
+    const float4 v = *reinterpret_cast<const float4*>(qg + gl * EPL);
+    q[0] = f2_pack(__float_as_uint(v.x), __float_as_uint(v.y));
+    q[1] = f2_pack(__float_as_uint(v.z), __float_as_uint(v.w));
+  }
+  const float sc2 = prm.att_scale * 1.4426950408889634f, sck = sc2 * qscale;  // scores in the log2 domain
+  float m = -INFINITY, l = 0.f;                            // l: this lane's share of the sum
+  uint64_t acc[NP2];
+#pragma unroll
+  for (int i = 0; i < NP2; ++i) acc[i] = 0ull;
+
+  // ---- the new token's own row, by the warp that would have the next tile ----
+  if (!prm.cached_new && gw == ntiles % nw) {
+    const float* src = prm.kv_new + (size_t)b * prm.kvn_stride + kvh * HD + lane * DPL;
+    float kv[2][DPL], qn[DPL], sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) { kv[0][i] = src[i]; kv[1][i] = src[prm.nkv * HD + i]; qn[i] = qg[lane * DPL + i]; }
+    float amax[2] = {0.f, 0.f};
+    if (KV_I8) {
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) amax[w] = fmaxf(amax[w], fabsf(kv[w][i]));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        amax[0] = fmaxf(amax[0], __shfl_xor_sync(0xffffffffu, amax[0], o));
+        amax[1] = fmaxf(amax[1], __shfl_xor_sync(0xffffffffu, amax[1], o));
+      }
+    }
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const size_t at = (crow0 + pos) * HD + lane * DPL;
+      if (KV_I8) {
+        const float scale = ((double)amax[w] > 1e-8) ? __fdiv_rn(amax[w], 127.0f) : 1.0f;
+        int8_t* c = static_cast<int8_t*>(w ? prm.v_cache : prm.k_cache) + at;
+        uint32_t bytes = 0;
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) {
+          const float r = fmaxf(-127.0f, fminf(127.0f, roundf(__fdiv_rn(kv[w][i], scale))));
+          const int8_t qv = (int8_t)r;
+          bytes |= (uint32_t)(uint8_t)qv << (8 * i);
+          kv[w][i] = __fmul_rn((float)qv, scale);
+        }
+        if (h % G == 0) {
+          if (DPL == 4) *reinterpret_cast<uint32_t*>(c) = bytes;
+          else *reinterpret_cast<uint16_t*>(c) = (uint16_t)bytes;
+          if (lane == 0) (w ? prm.v_scale : prm.k_scale)[crow0 + pos] = scale;
+        }
+      } else if (h % G == 0) {
+        float* c = static_cast<float*>(w ? prm.v_cache : prm.k_cache) + at;
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) c[i] = kv[w][i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) {
+      sum = fmaf(qn[i], kv[0][i], sum);
+      vn_s[lane * DPL + i] = kv[1][i];
+    }
+    m = warp_sum(sum) * sc2;
+    if (lane == 0) l = 1.f;  // 2^(m - m)
+    __syncwarp();
+    if (gi == 0) {
+#pragma unroll
+      for (int i = 0; i < NP2; ++i) acc[i] = *reinterpret_cast<const uint64_t*>(vn_s + gl * EPL + 2 * i);
+    }
+  }
+
+  // ---- cached rows ----
+  int s = 0;
+  uint32_t par = 0;
+#pragma unroll 1
+  for (int tile = gw; tile < ntiles; tile += nw) {
+    const int n = min(ROWS, cached - tile * ROWS);
+    float kc[NS], vc[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) { kc[i] = ksc[i]; vc[i] = vsc[i]; }
+    scales(tile + nw);
+    if (!__all_sync(0xffffffffu, mbar_wait(&full[warp][s], par))) {
+      if (lane == 0 && prm.error_flag) *reinterpret_cast<volatile int*>(prm.error_flag) = 1;
+      for (int i = 0; i < ATS_DEPTH && tile + i * nw < ntiles; ++i)  // the block outlives its copies in flight
+        mbar_wait(&full[warp][(s + i) % ATS_DEPTH], par ^ (uint32_t)(s + i >= ATS_DEPTH));
+      m = l = __int_as_float(0x7fc00000);
+      break;
+    }
+    const uint8_t* kt = ring + (size_t)s * 2 * ATS_TILE;
+    float d[ATS_PASSES];
+    if (KV_I8) {
+      // sixteen rows x 32 elements to an MMA; lane (g, t) reads bytes 16 t of every 64 of rows g and g + 8, and receives plane t of
+      // both; rows 2 .. ROWS / 8 such values are summed over the four lanes of g, the rows shared out among them
+      constexpr int MT = KV_I8 ? ROWS / 16 : 1;
+      const int g = lane >> 2, t = lane & 3;
+      const float wt = t < 3 ? __int_as_float((127 + 8 * t) << 23) : 0.f;  // 256^t
+      float v[2 * MT];
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        int c[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < HD / 64; ++j) {
+          const uint4 a = *reinterpret_cast<const uint4*>(kt + (16 * i + g) * ROWB + 64 * j + 16 * t);
+          const uint4 e = *reinterpret_cast<const uint4*>(kt + (16 * i + 8 + g) * ROWB + 64 * j + 16 * t);
+          imma_acc(c, a.x, e.x, a.y, e.y, qf[j].x, qf[j].y);
+          imma_acc(c, a.z, e.z, a.w, e.w, qf[j].z, qf[j].w);
+        }
+        v[2 * i] = wt * (float)c[0];
+        v[2 * i + 1] = wt * (float)c[2];
+      }
+      int n2 = 2 * MT;
+#pragma unroll
+      for (int o = 2; o > 0; o >>= 1) {
+        n2 >>= 1;
+        const bool up = (t & o) != 0;
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+          if (i < n2) {
+            const float keep = up ? v[i + n2] : v[i], give = up ? v[i] : v[i + n2];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < NS; ++i) d[i] = v[i];
+    } else {
+#pragma unroll
+      for (int u = 0; u < ATS_PASSES; ++u) {
+        const uint4 w = *reinterpret_cast<const uint4*>(kt + 512 * u + lane * 16);
+        float x, y;
+        f2_unpack(f2_fma(f2_pack(w.z, w.w), q[1], f2_mul(f2_pack(w.x, w.y), q[0])), x, y);
+        d[u] = x + y;
+      }
+      // sum over the LPP lanes of a row, the passes shared out among them
+      int cnt = ATS_PASSES;
+#pragma unroll
+      for (int o = LPP / 2; o > 0; o >>= 1) {
+        if (cnt > 1) {
+          cnt >>= 1;
+          const bool up = (gl & o) != 0;
+#pragma unroll
+          for (int i = 0; i < ATS_PASSES / 2; ++i)
+            if (i < cnt) {
+              const float keep = up ? d[i + cnt] : d[i], give = up ? d[i] : d[i + cnt];
+              d[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        } else {
+          d[0] += __shfl_xor_sync(0xffffffffu, d[0], o);
+        }
+      }
+    }
+    float mt = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      d[i] = row_of(i) < n ? d[i] * (kc[i] * sck) : -INFINITY;
+      mt = fmaxf(mt, d[i]);
+    }
+    const float mn = fmaxf(m, warp_max(mt));
+    const float alpha = exp2f(m - mn);
+    m = mn;
+    l *= alpha;
+    float pv[NS];
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      const float p = row_of(i) < n ? exp2f(d[i] - mn) : 0.f;
+      if (DUP == 1 || gl % DUP == 0) l += p;
+      pv[i] = p * vc[i];
+    }
+    const uint64_t al2 = f2_dup(alpha);
+#pragma unroll
+    for (int i = 0; i < NP2; ++i) acc[i] = f2_mul(acc[i], al2);
+#pragma unroll
+    for (int u = 0; u < ATS_PASSES; ++u) {
+      const uint4 w = *reinterpret_cast<const uint4*>(kt + ATS_TILE + 512 * u + lane * 16);
+      // the lane that holds the weight of row u RPP + gi
+      const int r = u * RPP + gi, from = KV_I8 ? 4 * (r & 7) + (r >> 3) / NS : gi * LPP + u * DUP;
+      const float p = __shfl_sync(0xffffffffu, pv[u % NS], from);
+      const uint64_t p2 = f2_dup(p);
+      if (KV_I8) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint64_t x, y;
+          ats_cvt4(u4_word(w, i), x, y);
+          acc[(2 * i) % NP2] = f2_fma(x, p2, acc[(2 * i) % NP2]);
+          acc[(2 * i + 1) % NP2] = f2_fma(y, p2, acc[(2 * i + 1) % NP2]);
+        }
+      } else {
+        const bool in = u * RPP + gi < n;  // bytes beyond the copy may spell a NaN
+        acc[0] = f2_fma(in ? f2_pack(w.x, w.y) : 0ull, p2, acc[0]);
+        acc[1 % NP2] = f2_fma(in ? f2_pack(w.z, w.w) : 0ull, p2, acc[1 % NP2]);
+      }
+    }
+    __syncwarp();
+    if (lane == 0 && tile + ATS_DEPTH * nw < ntiles) request(tile + ATS_DEPTH * nw, s);
+    if (++s == ATS_DEPTH) { s = 0; par ^= 1u; }
+  }
+  trace_stamp(rec, 5);
+
+  // ---- sum over the row groups, the dimensions shared out among them ----
+  float o[EPL];
+#pragma unroll
+  for (int i = 0; i < NP2; ++i) f2_unpack(acc[i], o[2 * i], o[2 * i + 1]);
+  int cnt = EPL, d0 = gl * EPL;
+#pragma unroll
+  for (int x = LPP; x < 32; x <<= 1) {
+    cnt >>= 1;
+    const bool up = (lane & x) != 0;
+#pragma unroll
+    for (int i = 0; i < EPL / 2; ++i)
+      if (i < cnt) {
+        const float keep = up ? o[i + cnt] : o[i], give = up ? o[i] : o[i + cnt];
+        o[i] = keep + __shfl_xor_sync(0xffffffffu, give, x);
+      }
+    if (up) d0 += cnt;
+  }
+  l = warp_sum(l);
+
+  // ---- every warp's result to the blocks that finish its dimensions ----
+  const int D = HD / C, to = d0 / D;
+  float* dst = part + gw * D + (d0 - to * D);
+  if (C > 1) {
+    cluster_wait();
+    const uint32_t a = cluster_map(smem_u32(dst), (uint32_t)to);
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a + 4 * i), "f"(o[i]) : "memory");
+    if (lane < C) {
+      const uint32_t c = cluster_map(smem_u32(&ml[gw]), (uint32_t)lane);
+      asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(c), "f"(m), "f"(l) : "memory");
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+  } else {
+#pragma unroll
+    for (int i = 0; i < DPL; ++i) dst[i] = o[i];
+    if (lane == 0) ml[gw] = make_float2(m, l);
+    __syncthreads();
+  }
+  trace_stamp(rec, 6);
+
+  // ---- this block's dimensions: D / ATS_WARPS per warp, the warps' results shared out among the lanes of a dimension ----
+  constexpr int WL = ATS_WARPS * ATS_MAX_CLUSTER / 32;  // warps of a cluster per lane
+  float2 e[WL];
+  float M = -INFINITY, L = 0.f, w[WL];
+#pragma unroll
+  for (int i = 0; i < WL; ++i) {
+    e[i] = 32 * i + lane < nw ? ml[32 * i + lane] : make_float2(-INFINITY, 0.f);
+    M = fmaxf(M, e[i].x);
+  }
+  M = warp_max(M);
+#pragma unroll
+  for (int i = 0; i < WL; ++i) {
+    w[i] = e[i].y == 0.f ? 0.f : exp2f(e[i].x - M);  // a warp without rows contributes nothing
+    L = fmaf(e[i].y, w[i], L);
+  }
+  const float inv = 1.0f / (warp_sum(L) + 1e-9f);
+  const int DW = D / ATS_WARPS, dim = warp * DW + lane % DW, g = lane / DW;
+  constexpr int PER = HD / 32;  // ATS_WARPS C results over 32 / DW lanes
+  float r = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int k = g * PER + i;
+    float f = __shfl_sync(0xffffffffu, w[0], k & 31);
+#pragma unroll
+    for (int j = 1; j < WL; ++j) {
+      const float fj = __shfl_sync(0xffffffffu, w[j], k & 31);
+      if (k >> 5 == j) f = fj;
+    }
+    r = fmaf(f, part[k * D + dim], r);
+  }
+  for (int x = DW; x < 32; x <<= 1) r += __shfl_xor_sync(0xffffffffu, r, x);
+  if (g == 0) prm.out[(size_t)b * prm.out_stride + h * HD + split * D + dim] = r * inv;
+  trace_stamp(rec, 7);
+}
+
+}  // namespace b200

@@ -11,8 +11,8 @@
 #include <memory>
 
 #include "attn.cuh"
-#include "attn_cluster.cuh"
 #include "attn_prefill.cuh"
+#include "attn_stream.cuh"
 #include "block_model.h"
 #include "dense_gemm.cuh"
 #include "dequant.cuh"
@@ -72,12 +72,12 @@ static void set_gemv_attrs() {
   CK(cudaFuncSetAttribute(gemv_batch_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
   CK(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_MAX));
   (void)tensor_map_encoder();
-  CK(cudaFuncSetAttribute((attn_decode_kernel<true, 0>), cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  CK(cudaFuncSetAttribute((attn_decode_kernel<false, 0>), cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  CK(cudaFuncSetAttribute((attn_decode_kernel<true, 64>), cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  CK(cudaFuncSetAttribute((attn_decode_kernel<false, 64>), cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  CK(cudaFuncSetAttribute((attn_decode_kernel<true, 128>), cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-  CK(cudaFuncSetAttribute((attn_decode_kernel<false, 128>), cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  CK(cudaFuncSetAttribute(attn_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  CK(cudaFuncSetAttribute(attn_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  CK(cudaFuncSetAttribute((attn_stream_kernel<true, 64>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ats_smem_bytes()));
+  CK(cudaFuncSetAttribute((attn_stream_kernel<false, 64>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ats_smem_bytes()));
+  CK(cudaFuncSetAttribute((attn_stream_kernel<true, 128>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ats_smem_bytes()));
+  CK(cudaFuncSetAttribute((attn_stream_kernel<false, 128>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ats_smem_bytes()));
   CK(cudaFuncSetAttribute((attn_prefill_kernel<true, 64>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pfa_smem_bytes(true, 64)));
   CK(cudaFuncSetAttribute((attn_prefill_kernel<true, 128>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pfa_smem_bytes(true, 128)));
   CK(cudaFuncSetAttribute((attn_prefill_kernel<false, 64>), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pfa_smem_bytes(false, 64)));
@@ -280,6 +280,19 @@ static size_t gemv_early_bytes() {
   return (size_t)kb * 1024;
 }
 
+static bool attn_stream_available(int hd, int nsplit) { return (hd == 64 || hd == 128) && (nsplit == 1 || nsplit == 2 || nsplit == 4 || nsplit == 8); }
+
+// Context splits per (sequence, head). attn_stream_kernel: a power of two up to the portable cluster size, at most as many blocks as there
+// are SMs (twice / four times as many, ms: 1.1B greedy 15.1 / 15.5 / 15.5, 1.1B with two sequences 12.3 / 12.4 / 13.7, 7B one sequence
+// 1.67 / 1.66 / 1.66, five 4.18 / 4.19 / 4.16: the launch after has to wait for them). Ticket kernel (head sizes 16 and 32): about four CTAs per SM.
+static int attn_nsplit(const b200_engine* e, int batch) {
+  const int heads = e->nq * batch;
+  if (!attn_stream_available(e->hd, 1)) return std::max(1, std::min((4 * e->num_sms + heads - 1) / heads, 32));
+  static const int per_sm = [] { const char* v = getenv("B200_ATTN_CTAS_PER_SM"); return v && atoi(v) > 0 ? atoi(v) : 1; }();
+  int c = 1;
+  while (2 * c * heads <= per_sm * e->num_sms && 2 * c <= ATS_MAX_CLUSTER) c *= 2;
+  return c;
+}
 static GvbLaunch gvb_launch(int K, const GemvSeg* seg, int nseg) {
   GvbLaunch l{K, 0, 0};
   for (int s = 0; s < nseg; ++s) {
@@ -396,32 +409,10 @@ static void launch_gemm_tc(const b200_engine* e, TcParams p, cudaStream_t st) {
   launch_pdl(e->use_pdl, gemm_tc_kernel, dim3(plan.grid), dim3(TC_THREADS), tc_smem_bytes(p.NT, p.bk, p.b_stages, p.w_stages, p.w_stage_bytes), st, p, maps);
 }
 
-// B200_ATTN_CLUSTER=1 runs the engine's attention as one thread-block cluster per head
-// (attn_cluster.cuh) instead of the ticket kernel; measured slower inside the step graph so far.
-static bool attn_use_cluster() {
-  static const bool on = [] { const char* v = getenv("B200_ATTN_CLUSTER"); return v && atoi(v) != 0; }();
-  return on;
-}
-
-// Context splits per (sequence, head): about four CTAs per SM for the ticket kernel; for the
-// cluster kernel a power of two up to 8 (the portable cluster size), about two CTAs per SM.
-static int attn_nsplit(const b200_engine* e, int batch) {
-  if (!attn_use_cluster()) {
-    static const int per_sm = [] { const char* v = getenv("B200_ATTN_CTAS_PER_SM"); return v && atoi(v) > 0 ? atoi(v) : 4; }();
-    int want = (per_sm * e->num_sms + e->nq * batch - 1) / (e->nq * batch);
-    return std::max(1, std::min(want, 32));
-  }
-  const int want = 2 * e->num_sms / std::max(1, e->nq * batch);
-  int cl = 1;
-  while (cl * 2 <= want && cl * 2 <= ATTC_MAX_CLUSTER) cl *= 2;
-  return cl;
-}
-
-// Starts decode attention: the cluster kernel when the split count is 1, 2, 4 or 8 (and the
-// ticket kernel is not forced), else the ticket kernel.
-static void launch_attention(const AttnParams& a, int batch, bool kv_i8, bool use_pdl, bool force_ticket, cudaStream_t st) {
+// Starts decode attention: head sizes 64 and 128 as one cluster of 1, 2, 4 or 8 splits per head, others (and other split counts) on the
+// ticket kernel.
+static void launch_attention(const AttnParams& a, int batch, bool kv_i8, bool use_pdl, cudaStream_t st) {
   const int ns = a.nsplit;
-  const bool cluster = !force_ticket && (ns == 1 || ns == 2 || ns == 4 || ns == 8);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ns, a.nq, batch);
   cfg.stream = st;
@@ -432,25 +423,24 @@ static void launch_attention(const AttnParams& a, int batch, bool kv_i8, bool us
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
   }
-  if (cluster) {
-    attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = ns;
-    attr[na].val.clusterDim.y = 1;
-    attr[na].val.clusterDim.z = 1;
-    ++na;
-    cfg.blockDim = dim3(ATTC_THREADS);
-    cfg.dynamicSmemBytes = attc_smem_floats(a.hd) * sizeof(float);
-    cfg.attrs = attr;
+  cfg.attrs = attr;
+  if (attn_stream_available(a.hd, ns)) {
+    if (ns > 1) {
+      attr[na].id = cudaLaunchAttributeClusterDimension;
+      attr[na].val.clusterDim.x = ns;
+      attr[na].val.clusterDim.y = 1;
+      attr[na].val.clusterDim.z = 1;
+      ++na;
+    }
     cfg.numAttrs = na;
+    cfg.blockDim = dim3(ATS_THREADS);
+    cfg.dynamicSmemBytes = ats_smem_bytes();
     if (a.hd == 128) {
-      if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_cluster_kernel<true, 128>, a));
-      else CK(cudaLaunchKernelEx(&cfg, attn_cluster_kernel<false, 128>, a));
-    } else if (a.hd == 64) {
-      if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_cluster_kernel<true, 64>, a));
-      else CK(cudaLaunchKernelEx(&cfg, attn_cluster_kernel<false, 64>, a));
+      if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_stream_kernel<true, 128>, a));
+      else CK(cudaLaunchKernelEx(&cfg, attn_stream_kernel<false, 128>, a));
     } else {
-      if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_cluster_kernel<true, 0>, a));
-      else CK(cudaLaunchKernelEx(&cfg, attn_cluster_kernel<false, 0>, a));
+      if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_stream_kernel<true, 64>, a));
+      else CK(cudaLaunchKernelEx(&cfg, attn_stream_kernel<false, 64>, a));
     }
     return;
   }
@@ -458,18 +448,9 @@ static void launch_attention(const AttnParams& a, int batch, bool kv_i8, bool us
   if (smem > 160 * 1024) throw std::runtime_error("context too long for the requested split count");
   cfg.blockDim = dim3(ATTN_GROUP_THREADS);
   cfg.dynamicSmemBytes = smem;
-  cfg.attrs = attr;
   cfg.numAttrs = na;
-  if (a.hd == 128) {
-    if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<true, 128>, a));
-    else CK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<false, 128>, a));
-  } else if (a.hd == 64) {
-    if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<true, 64>, a));
-    else CK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<false, 64>, a));
-  } else {
-    if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<true, 0>, a));
-    else CK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<false, 0>, a));
-  }
+  if (kv_i8) CK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<true>, a));
+  else CK(cudaLaunchKernelEx(&cfg, attn_decode_kernel<false>, a));
 }
 
 // Step-trace record of the launch with this index within the step (nullptr when tracing is off).
@@ -622,7 +603,7 @@ static int packed_forward_step(b200_engine* e, int batch, int nsplit, cudaStream
       AttnParams a{};
       fill_attn(a, nsplit);
       a.trace = trace_rec(e, launches);
-      launch_attention(a, batch, e->desc.kv_dtype == B200_KV_I8, e->use_pdl, !attn_use_cluster(), st);
+      launch_attention(a, batch, e->desc.kv_dtype == B200_KV_I8, e->use_pdl, st);
       ++launches;
     }
     {
@@ -772,7 +753,7 @@ static void prefill_chunk(b200_engine* e, int T, const std::vector<int>& meta, c
   const bool i8 = e->desc.kv_dtype == B200_KV_I8;
   embed_kernel<<<T, 256, 0, st>>>(d_tok, e->tok_embd.f32(), e->pf_h, H, e->V);
   CK(cudaGetLastError());
-  const int nsplit = attn_use_cluster() ? 1 : attn_nsplit(e, T);
+  const int nsplit = attn_nsplit(e, T);
   for (int l = 0; l < e->L; ++l) {
     const LayerW& w = e->layers[l];
     {
@@ -804,7 +785,7 @@ static void prefill_chunk(b200_engine* e, int T, const std::vector<int>& meta, c
       a.part_o = e->pf_part_o; a.part_ml = e->pf_part_ml; a.tickets = e->pf_tickets;
       a.out = e->pf_attn; a.out_stride = e->Hq; a.att_scale = 1.0f / std::sqrt((float)e->hd);
       a.cached_new = 1;
-      launch_attention(a, T, i8, false, true, st);
+      launch_attention(a, T, i8, false, st);
     }
     {
       GemvParams p{};

@@ -167,18 +167,6 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
 // the scale: scale * (q - off) = (128 scale) * X - (128 + off) * scale, X = 1 + q/128.
 __device__ __forceinline__ uint32_t byte_to_unit_float(uint32_t v, int k) { return __byte_perm(v, 0x3F000000u, 0x7044 | (k << 8)); }
 
-// Packed FP32 pairs (lower element in the low word).
-__device__ __forceinline__ uint64_t f2_pack(uint32_t lo, uint32_t hi) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-  return r;
-}
-__device__ __forceinline__ uint64_t f2_dup(float v) { return f2_pack(__float_as_uint(v), __float_as_uint(v)); }
-__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 __device__ __forceinline__ uint32_t f2_half2(uint64_t v) {
   uint32_t lo, hi;
   asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));

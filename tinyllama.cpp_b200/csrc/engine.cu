@@ -378,9 +378,6 @@ static void encode_map(CUtensorMap* tm, CUtensorMapDataType dt, int rank, const 
 static void launch_gemm_tc(const b200_engine* e, TcParams p, cudaStream_t st) {
   set_gemv_attrs();
   p.nblk = p.K / 256;
-  const int tiles_n0 = (p.T + TC_MAX_N - 1) / TC_MAX_N;
-  p.NT = ((p.T + tiles_n0 - 1) / tiles_n0 + 31) / 32 * 32;  // token tiles of equal width
-  p.tiles_n = (p.T + p.NT - 1) / p.NT;
   int tiles_m = 0, cell = 0;
   for (int s = 0; s < p.nseg; ++s) {
     tiles_m += (p.seg[s].rows + TC_M - 1) / TC_M;
@@ -389,8 +386,10 @@ static void launch_gemm_tc(const b200_engine* e, TcParams p, cudaStream_t st) {
   p.error_flag = e->d_error;
   p.ws = e->d_tc_part;
   p.tickets = e->d_tc_tickets;
-  const TcPlan plan = tc_plan(tiles_m * p.tiles_n, p.nblk, p.NT, e->num_sms, p.ws != nullptr);
+  const TcPlan plan = tc_plan(tiles_m, p.T, p.nblk, e->num_sms, p.ws != nullptr);
+  p.NT = plan.NT; p.tiles_n = plan.tiles_n;
   p.rem = plan.rem; p.ge = plan.ge; p.full = plan.full;
+  p.by_nblk = fast_div(p.nblk); p.by_tiles_n = fast_div(p.tiles_n); p.by_ge = fast_div(std::max(1, p.ge)); p.by_work = fast_div(std::max(1, p.rem * p.nblk));
   // shared memory: up to 128 KB of activation stages (a copy covers as many steps as 32 KB hold), the rest for packed units,
   // whose trip from HBM the kernel lives on when there are few tokens
   p.w_stage_bytes = 8 * cell;

@@ -4,24 +4,27 @@
 // (model.cpp:2141-2249). "Swap-AB": the weight rows are the M side of the MMA (128 per tile), the tokens
 // the N side (32..256 per tile).
 //
-// One persistent CTA (608 threads) per SM walks K block by block, four steps of 64 elements to a block:
+// One persistent CTA (640 threads) per SM walks K block by block, four steps of 64 elements to a block:
 //   * a weight-producer warp brings the packed units of the tile's 128 rows, one 256-element block at a time as eight
 //     contiguous cells (cp.async.bulk), into a ring;
-//   * sixteen warps dequantise into TENSOR MEMORY, which is where the MMA takes its A operand from:
-//     thread = (weight row = TMEM lane, one 64-element step of the block), 32 columns of packed fp16 pairs a
-//     step, two blocks; one wait, one fence and one arrival cover 64 elements of a thread;
+//   * sixteen warps dequantise into TENSOR MEMORY, which is where the MMA takes its A operand from: thread = (weight row =
+//     TMEM lane, half of a block), 64 columns of packed fp16 pairs. Two groups of eight warps take the blocks in turn, each
+//     with its own half of the weight columns, so that the waits and fences of one run under the conversions of the
+//     other (all sixteen on the same block: every phase of a block waited for the one before, 2200 cycles a block, 1900 now);
 //   * an activation-producer lane moves the matching slices of the fp16 activations with TMA
 //     (cp.async.bulk.tensor.3d, 128-byte swizzle, tokens beyond T read as zero), one to four steps a copy;
-//   * the MMA warp issues sixteen tcgen05.mma (M=128, N=NT, K=16, kind::f16) per block into an
-//     fp32 accumulator in tensor memory (two of them when NT <= 128). Its instruction stream is serial: as a
-//     branch for one lane, with two waits and a commit a step, it took 860 cycles a step, whatever NT, and everyone
-//     waited for it; so the warp runs it together, with few waits, and one lane is elected for the MMAs alone;
-//   * after a unit's last step the sixteen warps read their TMEM lanes back (tcgen05.ld 32x32b: thread =
-//     weight row, registers = tokens) and run the matvec kernel's epilogues.
-// Measured, 7B Q4_K shapes: a step of 16 sequences 8.3 ms with one CTA per tile and the fp16 tile in shared memory, 4.7 ms now;
-// a 1024-token prompt 32.7 and 23.1 ms. With few tokens the bound is issue: about 370 instructions per thread and
-// block, byte permutes at half rate, 1650 cycles a block and warp beside 1240 of MMA issue, where HBM would need 800. With 256
-// tokens it is the activation tiles: 128 KB a block and SM from L2, at about 36 bytes a cycle.
+//   * the MMA warp issues sixteen tcgen05.mma (M=128, N=NT, K=16, kind::f16) per block into an fp32 accumulator in tensor
+//     memory (two of them when NT <= 128). Alone it issues one in 21 cycles; beside busy warps each of its
+//     instructions waits its turn. So no branch of it depends on a wait, its operands are constants or loop counters (uniform
+//     registers), and it is one of the first warps;
+//   * after a unit's last step the sixteen warps read their TMEM lanes back (tcgen05.ld 32x32b: thread = weight row, registers
+//     = tokens) and run the matvec kernel's epilogues, each group's first block of the next unit being stored before.
+// Measured, ms, one CTA per tile and the fp16 tile in shared memory / all warps on one block / now: a step of 16 sequences of a 7B Q4_K
+// model 8.3 / 3.97 / 3.87, a 1024-token prompt 32.7 / 23.0 / 20.8; seven prompts of 1.1B 24.2 / 14.4 / 11.6. With few tokens the bound is the
+// dequantising warps (about 370 instructions per thread and block of 64 elements, byte permutes at half rate; fp16 pairs were tried: half of the
+// instructions for Q4_K, none for Q6_K, and results that depend on the token count), where HBM would need 800 cycles a
+// block; 10 us of a launch of 15 to 35 are its start, the hand-over of cut tiles and the epilogue. With 256 tokens it is the MMAs (2048 of
+// 2170 cycles a block) and the epilogue, which stores 32 bytes a cycle.
 // The roles meet on mbarriers only. Every wait is bounded; on a give-up the kernel sets the error word,
 // waits for its MMAs and copies, frees its tensor memory and returns.
 //
@@ -47,9 +50,20 @@ namespace b200 {
 
 constexpr int TC_M = 128;        // weight rows per CTA tile (the MMA's M)
 constexpr int TC_KC = 64;        // elements along K per step: one 128-byte swizzled row of fp16 activations
-constexpr int TC_WORKERS = 512;  // sixteen dequantising warps: thread = (weight row, 64-element quarter of a block)
-constexpr int TC_THREADS = TC_WORKERS + 96;  // + the MMA warp, the weight-producer warp and the activation-producer warp
+constexpr int TC_WORKERS = 512;  // sixteen dequantising warps in two groups that take blocks in turn: thread = (weight row, half of a block)
+constexpr int TC_GROUP = 8;      // warps of a group
+// Four service warps come first (MMA, weights, activations, tensor memory): a scheduler that holds a serial role and four busy warps
+// gives the lower number its turn.
+constexpr int TC_SERVICE = 4, TC_THREADS = TC_WORKERS + 32 * TC_SERVICE;
 constexpr int TC_MAX_N = 256;    // tokens per tile: half of the tensor memory holds accumulators, half the weight stages
+
+// floor(n / d) for n d < 2^38, n < 2^25: one multiplication (an integer division takes about 200 cycles, a unit of work a dozen of them)
+struct FastDiv {
+  unsigned long long m;
+  int d;
+};
+__host__ __device__ inline FastDiv fast_div(int d) { return {((1ull << 38) / (unsigned)d) + 1, d}; }
+__host__ __device__ __forceinline__ int operator/(int n, const FastDiv& f) { return (int)(((unsigned long long)(unsigned)n * f.m) >> 38); }
 
 struct TcParams {
   GemvSeg seg[3];
@@ -70,6 +84,7 @@ struct TcParams {
   const int* positions;           // [T]
   int head_dim, max_pos;
   int tiles_n;                    // token tiles; tile = row tile * tiles_n + token tile
+  FastDiv by_nblk, by_tiles_n, by_ge, by_work;  // of nblk, tiles_n, ge and rem * nblk
   int rem, ge, full;              // tiles 0 .. rem-1 are cut into ge ranges along K, the others run whole, `full` per CTA
   int bk, b_stages;               // steps of an activation stage (1, 2 or 4), stages
   int w_stages, w_stage_bytes;    // packed-weight ring: stages of eight cells
@@ -99,14 +114,19 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t leader, uint32_t tmem_d, uin
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
-// the same with A in tensor memory: lane = row, each 32-bit column two consecutive elements along K
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// 64 elements along K with A in tensor memory: lane = row, each 32-bit column two consecutive elements along K; 16 elements = 8 columns
+// of A, 32 bytes = 2 descriptor units of B
+__device__ __forceinline__ void tc_mma_f16_ts4(uint32_t leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(leader)
+      "setp.ne.b32 p, %8, 0;\n\t"
+      "setp.ne.b32 q, %9, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %5, %7, p;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], %6, %7, 1;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%3], %10, %7, 1;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%4], %11, %7, 1;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "r"(tmem_a + 8), "r"(tmem_a + 16), "r"(tmem_a + 24), "l"(desc_b), "l"(desc_b + 2), "r"(idesc), "r"(accumulate), "r"(leader),
+      "l"(desc_b + 4), "l"(desc_b + 6)
       : "memory");
 }
 // arrives on the mbarrier once every MMA issued so far by the leader has completed
@@ -179,55 +199,53 @@ __device__ __forceinline__ void tc_affine4(uint32_t bytes, uint64_t D, uint64_t 
   w1 = f2_half2(f2_fma(f2_pack(byte_to_unit_float(bytes, 2), byte_to_unit_float(bytes, 3)), D, C));
 }
 
-// The packed bytes one thread needs for its 64 elements [64 c, 64 c + 64) of a block, copied from the ring so that
+// The packed bytes one thread needs for its 128 elements [128 h, 128 h + 128) of a block, copied from the ring so that
 // the stage can be refilled while they are converted. cell, r: the row's cell and its row in it.
-//   Q4_K: r[0] = d, dmin, 12 scale bytes; r[1..2] = 32 nibble pairs (low nibbles = elements 0..31, high = 32..63)
-//   Q6_K: r[0..3] = ql bytes, r[4..5] = qh bytes of the 128-element half; aux = four sub-block scales; d = block scale
-//   Q8_0: r[0..3] = 64 quants; aux = two fp16 scales
+//   Q4_K: r[0] = d, dmin, 12 scale bytes; r[1..4] = nibble pairs, 32 bytes to 64 elements (low nibbles = elements 0..31, high = 32..63)
+//   Q6_K: r[0..3] = ql bytes, r[4..5] = qh bytes of the 128-element half; aux = eight sub-block scales; d = block scale
+//   Q8_0: r[0..7] = 128 quants; aux = four fp16 scales
 struct TcRaw {
-  uint4 r[6];
-  uint32_t aux;
+  uint4 r[8];
+  uint2 aux;
   uint16_t d;
 };
 
 template <int TYPE>
-__device__ __forceinline__ void tc_fetch(const uint8_t* cell, int r, int c, TcRaw& t) {
+__device__ __forceinline__ void tc_fetch(const uint8_t* cell, int r, int h, TcRaw& t) {
   const uint8_t* even = cell + 16 * r;                  // chunk 0 of the row; chunk n lies 256 n further,
   const uint8_t* odd = cell + 16 * (r ^ 4);             // odd chunks in the row's swapped place
   if (TYPE == T_Q4_K) {
     t.r[0] = *reinterpret_cast<const uint4*>(even);
-    t.r[1] = *reinterpret_cast<const uint4*>(odd + 256 * (1 + 2 * c));
-    t.r[2] = *reinterpret_cast<const uint4*>(even + 256 * (2 + 2 * c));
+#pragma unroll
+    for (int i = 1; i < 5; ++i) t.r[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + 256 * (4 * h + i));
   } else if (TYPE == T_Q6_K) {
-    const int hh = c >> 1;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t.r[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + 256 * (4 * hh + i));
+    for (int i = 0; i < 4; ++i) t.r[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + 256 * (4 * h + i));
 #pragma unroll
-    for (int i = 0; i < 2; ++i) t.r[4 + i] = *reinterpret_cast<const uint4*>((i ? odd : even) + 256 * (8 + 2 * hh + i));
-    t.aux = *reinterpret_cast<const uint32_t*>(even + 256 * 12 + 4 * c);
+    for (int i = 0; i < 2; ++i) t.r[4 + i] = *reinterpret_cast<const uint4*>((i ? odd : even) + 256 * (8 + 2 * h + i));
+    t.aux = *reinterpret_cast<const uint2*>(even + 256 * 12 + 8 * h);
     t.d = *reinterpret_cast<const uint16_t*>(cell + 16 * 208 + 2 * r);
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) t.r[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + 256 * (4 * c + i));
-    t.aux = *reinterpret_cast<const uint32_t*>(even + 256 * 16 + 4 * c);
+    for (int i = 0; i < 8; ++i) t.r[i] = *reinterpret_cast<const uint4*>(((i & 1) ? odd : even) + 256 * (8 * h + i));
+    t.aux = *reinterpret_cast<const uint2*>(even + 256 * 16 + 8 * h);
   }
 }
 
-// Half hf (32 elements) of the thread's 64 as sixteen fp16 pairs. Each weight is computed in FP32 as the reference
+// Elements 32 k .. 32 k + 31 (k < 4) of the thread's 128 as sixteen fp16 pairs; h: which half of the block they are. Each weight is computed in FP32 as the reference
 // does and rounded to fp16 once (scaling in fp16 pairs was measured to triple the error of the products: the sub-block
 // scale's rounding is shared by 16 or 32 weights and does not average out). Formulas: reference dequantize_q4_k_m /
 // dequantize_q6_k / dequantize_q8_0_block (quantization.cpp:171-266, 1047-1052). FP32 pairs (fma.rn.f32x2) halve the
 // multiply-adds; what is left per element is one byte permute and half a conversion.
 template <int TYPE>
-__device__ __forceinline__ void tc_dequant32(const TcRaw& t, int c, int hf, uint32_t (&w)[16]) {
+__device__ __forceinline__ void tc_dequant32(const TcRaw& t, int h, int k, uint32_t (&w)[16]) {
   if (TYPE == T_Q4_K) {
-    const uint4 h = t.r[0];
-    const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(&h.x));
-    // get_scale_min_k4 (quantization.cpp:145-155) of sub-block 2c + hf on the 12 scale bytes h.y h.z h.w
-    const int sh = 8 * (2 * (c & 1) + hf);
-    const uint32_t a = h.y >> sh, b = h.z >> sh, e = h.w >> sh;
-    const uint32_t sc = c < 2 ? (a & 63u) : ((e & 15u) | ((a >> 2) & 48u));
-    const uint32_t mn = c < 2 ? (b & 63u) : (((e >> 4) & 15u) | ((b >> 2) & 48u));
+    const uint4 hd = t.r[0];
+    const float2 dm = __half22float2(*reinterpret_cast<const __half2*>(&hd.x));
+    // get_scale_min_k4 (quantization.cpp:145-155) of sub-block 4h + k on the 12 scale bytes hd.y hd.z hd.w
+    const uint32_t a = hd.y >> (8 * k), b = hd.z >> (8 * k), e = hd.w >> (8 * k);
+    const uint32_t sc = h == 0 ? (a & 63u) : ((e & 15u) | ((a >> 2) & 48u));
+    const uint32_t mn = h == 0 ? (b & 63u) : (((e >> 4) & 15u) | ((b >> 2) & 48u));
     const float d1 = dm.x * (float)sc, m1 = dm.y * (float)mn;
     // d1 * q - m1 = D * X - (D + m1), D = 128 d1 (exact), X = 1 + q/128: the constant's rounding is 2^-24 of
     // 128 d1, far below the fp16 rounding of the result
@@ -235,32 +253,32 @@ __device__ __forceinline__ void tc_dequant32(const TcRaw& t, int c, int hf, uint
     const uint64_t D2 = f2_dup(D), C2 = f2_dup(-(D + m1));
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const uint32_t q = u4_word(t.r[1 + (i >> 2)], i & 3);
-      tc_affine4(((hf ? q >> 4 : q) & 0x0F0F0F0Fu) | 0x80808080u, D2, C2, w[2 * i], w[2 * i + 1]);
+      const uint32_t q = u4_word(t.r[1 + 2 * (k >> 1) + (i >> 2)], i & 3);
+      tc_affine4(((k & 1 ? q >> 4 : q) & 0x0F0F0F0Fu) | 0x80808080u, D2, C2, w[2 * i], w[2 * i + 1]);
     }
   } else if (TYPE == T_Q6_K) {
-    // 32-element group 2 (c & 1) + hf of the 128-element half: low nibbles of ql (high ones for the upper two groups),
+    // 32-element group k of the 128-element half: low nibbles of ql (high ones for the upper two groups),
     // two bits of qh brought to bits 4-5 by one rotation, one bitwise select, one more clears bits 6-7 and sets bit 7
     const float d = half_bits_to_float(t.d);
-    const int lsh = 4 * (c & 1), hrot = (4 - 2 * hf - 4 * (c & 1)) & 31;
+    const int lsh = 4 * (k >> 1), hrot = (4 - 2 * k) & 31;
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      const float sc = d * (float)(int)(int8_t)((t.aux >> (16 * hf + 8 * s)) & 0xFF);
+      const float sc = d * (float)(int)(int8_t)(((k >> 1 ? t.aux.y : t.aux.x) >> (16 * (k & 1) + 8 * s)) & 0xFF);
       const uint64_t D2 = f2_dup(128.0f * sc), C2 = f2_dup(-160.0f * sc);  // sc * (q - 32) = 128 sc * X - (128 + 32) sc
 #pragma unroll
       for (int i = 4 * s; i < 4 * s + 4; ++i) {
-        const uint32_t lo = u4_word(t.r[2 * hf + (i >> 2)], i & 3) >> lsh, hw = u4_word(t.r[4 + (i >> 2)], i & 3);
+        const uint32_t lo = u4_word(t.r[2 * (k & 1) + (i >> 2)], i & 3) >> lsh, hw = u4_word(t.r[4 + (i >> 2)], i & 3);
         const uint32_t hi = __funnelshift_l(hw, hw, hrot);
         tc_affine4(((((lo ^ hi) & 0x0F0F0F0Fu) ^ hi) & 0x3F3F3F3Fu) | 0x80808080u, D2, C2, w[2 * i], w[2 * i + 1]);
       }
     }
   } else {
     // 0x4B0000bb is 8388608 + bb; the pairs' subtraction and product are exact, the one rounding is that to fp16
-    const float d = scale_field_to_float((uint16_t)((t.aux >> (16 * hf)) & 0xFFFF));
+    const float d = scale_field_to_float((uint16_t)(((k >> 1 ? t.aux.y : t.aux.x) >> (16 * (k & 1))) & 0xFFFF));
     const uint64_t one = f2_dup(1.0f), off = f2_dup(-8388736.0f), D2 = f2_dup(d), zero = f2_dup(0.0f);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const uint32_t q = u4_word(t.r[2 * hf + (i >> 2)], i & 3) ^ 0x80808080u;  // int8 + 128 as an unsigned byte
+      const uint32_t q = u4_word(t.r[2 * k + (i >> 2)], i & 3) ^ 0x80808080u;  // int8 + 128 as an unsigned byte
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
         const uint64_t x = f2_pack(__byte_perm(q, 0x4B000000u, 0x7440 | (2 * k)), __byte_perm(q, 0x4B000000u, 0x7440 | (2 * k + 1)));
@@ -279,14 +297,14 @@ struct alignas(64) TcMaps {
 };
 
 struct TcShared {
-  unsigned long long a_full[2];              // the sixteen warps have stored a block's weights
+  unsigned long long a_full[2];              // a group's warps have stored a block's weights
   unsigned long long a_empty[2];             // the MMAs that read them have completed
   unsigned long long b_full[TC_B_STAGES];    // the activation tile has landed (TMA transaction bytes)
   unsigned long long b_empty[TC_B_STAGES];   // the MMAs that read it have completed
   unsigned long long acc_full[2];            // all MMAs of a unit have completed
   unsigned long long acc_empty[2];           // the sixteen warps have read the accumulator
   unsigned long long w_full[TC_W_STAGES];    // the packed units of a block have landed
-  unsigned long long w_empty[TC_W_STAGES];   // the sixteen warps have copied their part of the stage into registers
+  unsigned long long w_empty[TC_W_STAGES];   // a group's warps have copied their part of the stage into registers
   unsigned long long drained;                // all MMAs issued by this CTA have completed
   uint32_t tmem_base;
   int abort_flag;
@@ -339,30 +357,44 @@ __host__ __device__ __forceinline__ size_t tc_smem_bytes(int NT, int bk, int b_s
 }
 constexpr int TC_SMEM_MAX = 226 * 1024;  // dynamic part; the barriers live in static shared memory
 
-// How `tiles` tiles of nblk blocks fall to `sms` CTAs: whole waves, and the tiles left over cut into ge ranges along K.
+// How a launch is cut: token tiles of NT; whole waves of tiles, and the tiles left over cut into ge ranges along K.
 struct TcPlan {
-  int rem, ge, full, grid;
+  int NT, tiles_n, rem, ge, full, grid;
+  double cost;  // cycles
 };
-inline TcPlan tc_plan(int tiles, int nblk, int NT, int sms, bool cut) {
-  TcPlan r;
-  r.full = tiles / sms;
-  r.rem = tiles - r.full * sms;
-  r.ge = r.rem;
-  if (r.rem && cut) {
-    // Cycles: a block takes four steps, each bound by the MMAs (2 NT cycles) or by dequantisation (about 250); a cut tile's
-    // sums travel to the workspace and back at about 32 bytes a cycle, read by its last CTA, behind a ticket (about 1500).
-    const double block = 4.0 * std::max(2 * NT, 250), part = NT * 128 * 4 / 32.0;
-    double best = block * nblk;
-    for (int k = 2; ; ++k) {
-      const int ge = std::min({k * r.rem, sms, r.rem * nblk});
-      const double t = block * ((r.rem * nblk + ge - 1) / ge) + part * ((ge + r.rem - 1) / r.rem + 1) + 1500;
-      if (t < best) { best = t; r.ge = ge; }
-      if (ge < k * r.rem) break;
-      if (ge == sms || ge == r.rem * nblk) break;
+// The cheapest width of token tiles and cut of the last wave, in cycles as measured (7B and 1.1B Q4_K, 16 to 512 tokens): a block costs 1900
+// (dequantisation) or, from 224 tokens on, 8.6 a token (MMAs, activations from L2); a tile's epilogue 16 a token (stores leave an
+// SM at 32 bytes a cycle) and 800; a cut tile's parts are written (16 a token, 1.5 of them a CTA), met (3000) and read by the last CTA (8 a
+// token each). Always 256 tokens to a tile took, 512 tokens, cycles: 1.1B O 30000 / 20000 (64), 7B O 45000 / 38000 (128).
+inline TcPlan tc_plan(int tiles_m, int T, int nblk, int sms, bool cut) {
+  TcPlan best{};
+  int last = 0;
+  for (int tn = (T + TC_MAX_N - 1) / TC_MAX_N; tn <= (T + 31) / 32; ++tn) {
+    TcPlan r{};
+    r.NT = ((T + tn - 1) / tn + 31) / 32 * 32;
+    if (r.NT == last) continue;
+    last = r.NT;
+    r.tiles_n = (T + r.NT - 1) / r.NT;
+    const int tiles = tiles_m * r.tiles_n;
+    const double block = std::max(1900.0, 8.6 * r.NT), epi = 16.0 * r.NT + 800, whole = nblk * block + epi;
+    r.full = tiles / sms;
+    r.rem = tiles - r.full * sms;
+    r.ge = r.rem;
+    r.cost = r.full * whole;
+    if (r.rem) {
+      double t = whole;
+      for (int k = 2; cut; ++k) {
+        const int ge = std::min({k * r.rem, sms, r.rem * nblk});
+        const double c = block * ((r.rem * nblk + ge - 1) / ge) + 1.5 * 16 * r.NT + 3000 + ((ge + r.rem - 1) / r.rem + 1) * 8.0 * r.NT + epi;
+        if (c < t) { t = c; r.ge = ge; }
+        if (ge < k * r.rem || ge == sms || ge == r.rem * nblk) break;
+      }
+      r.cost += t;
     }
+    r.grid = r.full ? sms : r.ge;
+    if (!best.NT || r.cost < best.cost) best = r;
   }
-  r.grid = r.full ? sms : r.ge;
-  return r;
+  return best;
 }
 
 // Workspace of an engine: two parts of a 128 x 256 tile per CTA.
@@ -377,15 +409,15 @@ __device__ __forceinline__ bool tc_work(const TcParams& p, int cta, int i, TcWor
   w.c0 = w.c1 = cta;
   bool cut = false;
   if (cta < p.ge) {
-    const int W = p.rem * p.nblk, x0 = cta * W / p.ge, x1 = (cta + 1) * W / p.ge;  // at most nblk blocks: one or two tiles
-    const int a = x0 / p.nblk, mid = min(x1, (a + 1) * p.nblk);
+    const int W = p.rem * p.nblk, x0 = cta * W / p.by_ge, x1 = (cta + 1) * W / p.by_ge;  // at most nblk blocks: one or two tiles
+    const int a = x0 / p.by_nblk, mid = min(x1, (a + 1) * p.nblk);
     const int two = x1 > mid;
     if (i <= two) {
       w.tile = a + i;
       w.b0 = i ? 0 : x0 - a * p.nblk;
       w.nb = i ? x1 - mid : mid - x0;
-      w.c0 = ((w.tile * p.nblk + 1) * p.ge - 1) / W;
-      w.c1 = ((w.tile + 1) * p.nblk * p.ge - 1) / W;
+      w.c0 = ((w.tile * p.nblk + 1) * p.ge - 1) / p.by_work;
+      w.c1 = ((w.tile + 1) * p.nblk * p.ge - 1) / p.by_work;
       cut = true;
     }
     i -= 1 + two;
@@ -396,7 +428,7 @@ __device__ __forceinline__ bool tc_work(const TcParams& p, int cta, int i, TcWor
     w.b0 = 0;
     w.nb = p.nblk;
   }
-  int m = w.tile / p.tiles_n;
+  int m = w.tile / p.by_tiles_n;
   w.t0 = (w.tile - m * p.tiles_n) * p.NT;
   w.seg = 0;
   while (w.seg + 1 < p.nseg && m >= (p.seg[w.seg].rows + TC_M - 1) / TC_M) { m -= (p.seg[w.seg].rows + TC_M - 1) / TC_M; ++w.seg; }
@@ -404,99 +436,193 @@ __device__ __forceinline__ bool tc_work(const TcParams& p, int cta, int i, TcWor
   return true;
 }
 // Workspace slot of CTA c's part of a cut tile (a CTA has a part of at most two).
-__device__ __forceinline__ int tc_slot(const TcParams& p, int c, int tile) { return 2 * c + (c * (p.rem * p.nblk) / p.ge / p.nblk != tile); }
+__device__ __forceinline__ int tc_slot(const TcParams& p, int c, int tile) { return 2 * c + (c * (p.rem * p.nblk) / p.by_ge / p.by_nblk != tile); }
 
-// Eight finished columns (tokens t .. t+7) of this lane's row: the epilogue.
-__device__ __forceinline__ void tc_finish8(const TcParams& p, const TcWork& w, int row, int t, const float (&v)[8]) {
-  const int lane = threadIdx.x & 31;
+// ---- epilogue ----
+// A warp's columns (tokens c_begin .. c_end - 1 of the tile) of its 32 rows, eight at a time, from tensor memory or, CUT, as the sum of a
+// cut tile's parts. Stores leave an SM at 32 bytes a cycle whatever their form (measured: 4-byte, 16-byte and bulk), 4100 cycles for a
+// 256-token tile of FP32 whose products take 37000, and with one accumulator no MMA runs meanwhile. So each kind of epilogue has a loop
+// of its own (with one for all kinds such a tile took 9000 to 13000), a group's reads (residual, rotation) are requested a group ahead, the
+// first ones before the accumulator is complete, and both lanes of a gate / up pair work.
+template <int EPI, bool CUT>
+__device__ __forceinline__ void tc_drain(const TcParams& p, TcShared& sh, const TcWork& w, uint32_t acc, void* full, uint32_t parity) {
+  const int warp = (threadIdx.x >> 5) - TC_SERVICE, lane = threadIdx.x & 31, r = 32 * (warp & 3) + lane, row = w.row0 + r;
+  const int q_cols = p.NT / 4, c_begin = (warp >> 2) * q_cols, c_end = min(c_begin + q_cols, p.T - w.t0);  // NT is a multiple of 32
   const bool row_ok = row < p.seg[w.seg].rows;
-  const int n = min(8, p.T - t);
-  if (p.epi == EPI_SWIGLU) {
-    // image rows: eight gate rows then the same eight up rows (reference model.cpp:734-735, batch form
-    // cpu_batch_processor.cpp:252-256: (g / (1 + exp(-g))) * u)
-    const size_t at = (size_t)t * p.y_stride + (row >> 4) * 8 + (row & 7);
+  const size_t ld = EPI == EPI_QKV_ROPE && w.seg > 0 ? p.y2_stride : p.y_stride;
+  const bool upper = EPI == EPI_SWIGLU && (row & 8);
+  size_t at = (size_t)(w.t0 + c_begin) * ld;
+  float* y = p.y;
+  if (EPI == EPI_QKV_ROPE) {
+    if (w.seg > 0) y = p.y2 + (w.seg == 2 ? p.seg[1].rows : 0);
+    at += row;
+  } else if (EPI == EPI_SWIGLU) {
+    at += (row >> 4) * 8 + (row & 7) + (upper ? ld : 0);  // the gate lane takes the even tokens, the up lane the odd ones
+  } else {
+    at += row;
+  }
+  const float* res = (EPI == EPI_RESID && p.resid ? p.resid : y) + at;
+  const int i = EPI == EPI_QKV_ROPE ? (row % p.head_dim) >> 1 : 0;
+  float2 a[8];  // RESID: the residual (x); QKV: cosine and sine, or (2, 0): the row is not rotated
+  auto ahead = [&](int c0) {
+    if (EPI == EPI_RESID) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float up = __shfl_sync(0xffffffffu, v[j], (lane & 23) + 8);
-      if (row_ok && !(row & 8) && j < n) {
-        const float o = (v[j] / (1.0f + expf(-v[j]))) * up;
-        if (p.y16) p.y16[at + (size_t)j * p.y_stride] = __float2half_rn(o);
-        else p.y[at + (size_t)j * p.y_stride] = o;
+      for (int j = 0; j < 8; ++j) a[j].x = row_ok && c0 + j < c_end ? res[j * ld] : 0.f;
+      res += 8 * ld;
+    } else if (EPI == EPI_QKV_ROPE) {
+      const int mine = w.seg < 2 && lane < 8 && c0 + lane < c_end ? p.positions[w.t0 + c0 + lane] : -1;  // lane j: the position of token j
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int pos = __shfl_sync(0xffffffffu, mine, j);
+        a[j] = pos >= 0 && pos < p.max_pos ? *reinterpret_cast<const float2*>(p.rope + ((size_t)pos * (p.head_dim >> 1) + i) * 2) : make_float2(2.f, 0.f);
       }
     }
-  } else if (p.epi == EPI_RESID) {
-    if (!row_ok) return;
-    const float* rs = (p.resid ? p.resid : p.y) + (size_t)t * p.y_stride + row;
-    float* y = p.y + (size_t)t * p.y_stride + row;
-    float r[8];
+  };
+  if (c_begin < c_end) ahead(c_begin);
+  if (!CUT) {
+    tc_wait(p, &sh, full, parity);
+    __syncwarp();
+    tc_fence_after();
+  }
+#pragma unroll 1
+  for (int c0 = c_begin; c0 < c_end; c0 += 8, at += 8 * ld) {
+    float v[8];
+    if (CUT) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) r[j] = j < n ? rs[(size_t)j * p.y_stride] : 0.f;
+      for (int j = 0; j < 8; ++j) v[j] = 0.f;
+#pragma unroll 2
+      for (int c = w.c0; c <= w.c1; ++c) {
+        const float* src = p.ws + ((size_t)tc_slot(p, c, w.tile) * p.NT + c0) * TC_M + r;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (j < n) y[(size_t)j * p.y_stride] = r[j] + v[j];
-  } else if (p.epi == EPI_QKV_ROPE) {
-    const int i = (row % p.head_dim) >> 1;
-    float* y = w.seg == 0 ? p.y + (size_t)t * p.y_stride + row : p.y2 + (size_t)t * p.y2_stride + (w.seg == 2 ? p.seg[1].rows : 0) + row;
-    const int ld = w.seg == 0 ? p.y_stride : p.y2_stride;
-    float2 cs[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int pos = w.seg < 2 && j < n ? p.positions[t + j] : -1;
-      cs[j] = pos >= 0 && pos < p.max_pos ? *reinterpret_cast<const float2*>(p.rope + ((size_t)pos * (p.head_dim >> 1) + i) * 2) : make_float2(2.f, 0.f);
+        for (int j = 0; j < 8; ++j) v[j] += __ldcg(src + (size_t)j * TC_M);
+      }
+    } else {
+      tc_ld8(acc + (uint32_t)c0, v);
     }
+    if (EPI == EPI_SWIGLU) {
+      // image rows: eight gate rows then the same eight up rows (reference model.cpp:734-735, batch form
+      // cpu_batch_processor.cpp:252-256: (g / (1 + exp(-g))) * u)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float other = __shfl_xor_sync(0xffffffffu, v[j], 1);
-      float o = v[j];
-      if (cs[j].x < 1.5f)  // a cosine: the row is rotated
-        o = (row & 1) ? __fadd_rn(__fmul_rn(other, cs[j].y), __fmul_rn(v[j], cs[j].x)) : __fsub_rn(__fmul_rn(v[j], cs[j].x), __fmul_rn(other, cs[j].y));
-      if (row_ok && j < n) y[(size_t)j * ld] = o;
+      for (int j = 0; j < 8; j += 2) {
+        const float got = __shfl_xor_sync(0xffffffffu, upper ? v[j] : v[j + 1], 8);
+        const float g = upper ? got : v[j], u = upper ? v[j + 1] : got;
+        const float o = (g / (1.0f + expf(-g))) * u;
+        if (row_ok && c0 + j + (upper ? 1 : 0) < c_end) {
+          if (p.y16) p.y16[at + j * ld] = __float2half_rn(o);
+          else y[at + j * ld] = o;
+        }
+      }
+    } else {
+      if (EPI == EPI_RESID) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = a[j].x + v[j];
+      } else if (EPI == EPI_QKV_ROPE) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float other = __shfl_xor_sync(0xffffffffu, v[j], 1);
+          if (a[j].x < 1.5f)  // a cosine: the row is rotated
+            v[j] = (row & 1) ? __fadd_rn(__fmul_rn(other, a[j].y), __fmul_rn(v[j], a[j].x)) : __fsub_rn(__fmul_rn(v[j], a[j].x), __fmul_rn(other, a[j].y));
+        }
+      }
+      if (c0 + 8 < c_end) ahead(c0 + 8);
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (row_ok && c0 + j < c_end) y[at + j * ld] = v[j];
     }
-  } else if (row_ok) {
-    float* y = p.y + (size_t)t * p.y_stride + row;
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (j < n) y[(size_t)j * p.y_stride] = v[j];
   }
 }
+template <bool CUT>
+__device__ __forceinline__ void tc_drain(const TcParams& p, TcShared& sh, const TcWork& w, uint32_t acc, void* full, uint32_t parity) {
+  if (p.epi == EPI_SWIGLU) tc_drain<EPI_SWIGLU, CUT>(p, sh, w, acc, full, parity);
+  else if (p.epi == EPI_RESID) tc_drain<EPI_RESID, CUT>(p, sh, w, acc, full, parity);
+  else if (p.epi == EPI_QKV_ROPE) tc_drain<EPI_QKV_ROPE, CUT>(p, sh, w, acc, full, parity);
+  else tc_drain<EPI_STORE, CUT>(p, sh, w, acc, full, parity);
+}
 
-// One unit's blocks by a dequantising warp; blk: blocks of this CTA before it (ring position).
+// Where a dequantising warp stands: its group's next block, counted over the CTA's units, and that block's stage of the ring.
+struct TcStand {
+  int blk, stage;
+  uint32_t par;
+};
+
+// The group's blocks below `end` (all of type TYPE).
 template <int TYPE>
-__device__ __forceinline__ void tc_dequant_unit(const TcParams& p, TcShared& sh, const uint8_t* Wbase, uint32_t tmem, const TcWork& w, int blk) {
+__device__ __forceinline__ void tc_dequant_to(const TcParams& p, TcShared& sh, const uint8_t* Wbase, uint32_t tmem, TcStand& at, int end) {
   constexpr int cell = TYPE == T_Q4_K ? 16 * 144 : TYPE == T_Q6_K ? 16 * 208 + 32 : 16 * 272;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int my_row = threadIdx.x & (TC_M - 1), c = warp >> 2;
-  const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
-  int stage = blk % p.w_stages;
-  uint32_t wpar = (uint32_t)((blk / p.w_stages) & 1);
+  const int warp = (threadIdx.x >> 5) - TC_SERVICE, lane = threadIdx.x & 31, group = warp / TC_GROUP, h = (warp >> 2) & 1;
+  const int my_row = threadIdx.x & (TC_M - 1);
+  const uint32_t dst = tmem + TC_A_COL + 128u * (uint32_t)group + 64u * (uint32_t)h + ((uint32_t)(32 * (warp & 3)) << 16);
 #pragma unroll 1
-  for (int i = 0; i < w.nb; ++i, ++blk) {
-    tc_wait(p, &sh, &sh.w_full[stage], wpar);
+  for (; at.blk < end; at.blk += 2) {
+    const int stage = at.stage, blk = at.blk;
+    tc_wait(p, &sh, &sh.w_full[stage], at.par);
+    for (int i = 0; i < 2; ++i)
+      if (++at.stage == p.w_stages) { at.stage = 0; at.par ^= 1u; }
     TcRaw raw;
-    tc_fetch<TYPE>(Wbase + (size_t)stage * p.w_stage_bytes + (size_t)(my_row >> 4) * cell, my_row & 15, c, raw);
+    tc_fetch<TYPE>(Wbase + (size_t)stage * p.w_stage_bytes + (size_t)(my_row >> 4) * cell, my_row & 15, h, raw);
     uint32_t v[16];
-    tc_dequant32<TYPE>(raw, c, 0, v);
+    tc_dequant32<TYPE>(raw, h, 0, v);
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh.w_empty[stage]);  // the stage may be refilled
-    if (++stage == p.w_stages) { stage = 0; wpar ^= 1u; }
     // the MMAs that read this half of the weight columns two blocks ago must be done before it is overwritten
-    const int sa = blk & 1;
-    if (blk >= 2) tc_wait(p, &sh, &sh.a_empty[sa], (uint32_t)(((blk >> 1) - 1) & 1));
+    if (blk >= 2) tc_wait(p, &sh, &sh.a_empty[group], (uint32_t)(((blk >> 1) - 1) & 1));
     tc_fence_after();
-    const uint32_t dst = tmem + TC_A_COL + 32u * (uint32_t)(4 * sa + c) + lanes;
     __syncwarp();
     tc_st16(dst, v);
-    tc_dequant32<TYPE>(raw, c, 1, v);
-    tc_st16(dst + 16, v);
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+      tc_dequant32<TYPE>(raw, h, k, v);
+      tc_st16(dst + 16 * k, v);
+    }
     tc_wait_st();
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sh.a_full[sa]);
+    if (lane == 0) mbar_arrive(&sh.a_full[group]);
   }
 }
 
-// grid: tc_plan. 608 threads: warps 0-15 dequantise and run the epilogue, warp 16 issues the MMAs, warp 17
-// moves the packed weights, warp 18 the activation tiles. A programmatic dependent launch: only the activation producer and
+// The sums of unit u (finished by its last MMA) out of tensor memory: a warp holds lanes 32 * (warp & 3) .. +31 (= weight rows), the
+// four warps of equal rows split the tokens.
+__device__ __forceinline__ void tc_epilogue(const TcParams& p, TcShared& sh, uint32_t tmem, const TcWork& w, int u, int nbuf) {
+  const int warp = (threadIdx.x >> 5) - TC_SERVICE, lane = threadIdx.x & 31;
+  const int buf = nbuf == 2 ? (u & 1) : 0, use = nbuf == 2 ? (u >> 1) : u;
+  const uint32_t acc = tmem + 128u * (uint32_t)buf + ((uint32_t)(32 * (warp & 3)) << 16), parity = (uint32_t)(use & 1);
+  if (u == 0) pdl_wait();
+  const bool whole = w.c0 == w.c1;
+  if (whole) {
+    tc_drain<false>(p, sh, w, acc, &sh.acc_full[buf], parity);
+  } else {
+    const int q_cols = p.NT / 4, c_begin = (warp >> 2) * q_cols, c_end = min(c_begin + q_cols, p.T - w.t0);
+    float* part = p.ws + ((size_t)tc_slot(p, blockIdx.x, w.tile) * p.NT + c_begin) * TC_M + 32 * (warp & 3) + lane;
+    tc_wait(p, &sh, &sh.acc_full[buf], parity);
+    __syncwarp();
+    tc_fence_after();
+#pragma unroll 1
+    for (int c0 = c_begin; c0 < c_end; c0 += 8, part += 8 * TC_M) {
+      float v[8];
+      tc_ld8(acc + (uint32_t)c0, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) __stcg(part + j * TC_M, v[j]);
+    }
+  }
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(&sh.acc_empty[buf]);
+  if (whole) return;
+  __threadfence();
+  tc_workers_sync();
+  if (threadIdx.x == 32 * TC_SERVICE) {
+    sh.last = atomicAdd(&p.tickets[w.tile], 1) == w.c1 - w.c0;
+    if (sh.last) p.tickets[w.tile] = 0;
+    __threadfence();
+  }
+  tc_workers_sync();
+  if (sh.last != 0) tc_drain<true>(p, sh, w, 0u, nullptr, 0u);
+  tc_workers_sync();  // sh.last is read before the next unit writes it
+}
+
+// grid: tc_plan. 640 threads: warp 0 issues the MMAs, warp 1 moves the packed weights, warp 2 the activation tiles, warp 3 holds the tensor
+// memory, warps 4-19 dequantise and run the epilogue. A programmatic dependent launch: only the activation producer and
 // the epilogue wait for the previous kernel; weights are fetched and dequantised ahead of it.
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_constant__ TcParams p, const __grid_constant__ TcMaps maps) {
   extern __shared__ uint8_t tc_smem_raw[];
@@ -507,70 +633,70 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
   uint8_t* const Wbase = Bbase + (size_t)p.b_stages * b_stage_bytes;  // [w_stages][128 rows][unit bytes]
   const int nbuf = p.NT <= (int)TC_A_COL / 2 ? 2 : 1;                 // accumulators, 128 columns apart
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&sh.a_full[i], TC_WORKERS / 32); mbar_init(&sh.a_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&sh.a_full[i], TC_GROUP); mbar_init(&sh.a_empty[i], 1); }
     for (int i = 0; i < TC_B_STAGES; ++i) { mbar_init(&sh.b_full[i], 1); mbar_init(&sh.b_empty[i], 1); }
-    for (int i = 0; i < TC_W_STAGES; ++i) { mbar_init(&sh.w_full[i], 1); mbar_init(&sh.w_empty[i], TC_WORKERS / 32); }
+    for (int i = 0; i < TC_W_STAGES; ++i) { mbar_init(&sh.w_full[i], 1); mbar_init(&sh.w_empty[i], TC_GROUP); }
     for (int i = 0; i < 2; ++i) { mbar_init(&sh.acc_full[i], 1); mbar_init(&sh.acc_empty[i], TC_WORKERS / 32); }
     mbar_init(&sh.drained, 1);
     sh.abort_flag = 0;
     sh.w_issued = sh.b_issued = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) tc_alloc(&sh.tmem_base, 512);
+  if (warp == 3) tc_alloc(&sh.tmem_base, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   pdl_launch_dependents();
-  const uint32_t tmem = sh.tmem_base;
+  // All 512 columns: the allocation starts at column 0, which keeps the MMAs' operands constants (uniform registers) instead of loads
+  constexpr uint32_t tmem = 0;
+  if (sh.tmem_base != tmem && tid == 0) {
+    sh.abort_flag = 1;
+    if (p.error_flag) *reinterpret_cast<volatile int*>(p.error_flag) = 1;
+  }
   TcWork w;
 
-  if (warp == TC_WORKERS / 32) {
+  if (warp == 0) {
     // ---- MMA warp ----
     const uint32_t leader = warp_leader();
     const uint32_t idesc = tc_idesc(p.NT);
     const uint64_t bdesc0 = tc_smem_desc(smem_u32(Bbase)), b_step = (uint64_t)((p.NT * 128) >> 4);
     int sb = 0, blk = 0;
     uint32_t pb = 0;
-    uint64_t bdesc = bdesc0;
-    bool ok = true;
-    auto wait = [&](void* bar, uint32_t parity) { return __all_sync(0xffffffffu, tc_wait(p, &sh, bar, parity)) != 0; };
-    for (int u = 0; ok && tc_work(p, blockIdx.x, u, w); ++u) {
+    // No branch depends on a wait: the loops stay uniform over the warp. After a give-up the waits return at once, the MMAs run on
+    // what is there, and the results are dropped by the error word.
+    for (int u = 0; tc_work(p, blockIdx.x, u, w); ++u) {
       const int buf = nbuf == 2 ? (u & 1) : 0, use = nbuf == 2 ? (u >> 1) : u;
-      if (use > 0 && !(ok = wait(&sh.acc_empty[buf], (uint32_t)((use - 1) & 1)))) break;
+      if (use > 0) tc_wait(p, &sh, &sh.acc_empty[buf], (uint32_t)((use - 1) & 1));
       const uint32_t d = tmem + 128u * (uint32_t)buf;
-      uint32_t accumulate = 0;
 #pragma unroll 1
       for (int i = 0; i < w.nb; ++i, ++blk) {
         const int sa = blk & 1;
-        if (!(ok = wait(&sh.a_full[sa], (uint32_t)((blk >> 1) & 1)))) break;
-        uint32_t a = tmem + TC_A_COL + 128u * (uint32_t)sa;
-#pragma unroll 1
-        for (int k = 0; k < 4; k += p.bk) {
-          if (!(ok = wait(&sh.b_full[sb], pb))) break;
-          tc_fence_after();
-#pragma unroll 1
-          for (int j = 0; j < p.bk; ++j) {
-            tc_mma_f16_ts(leader, d, a, bdesc, idesc, accumulate);  // 16 elements along K = 8 columns of A, 32 bytes = 2 descriptor units of B
-            tc_mma_f16_ts(leader, d, a + 8, bdesc + 2, idesc, 1u);
-            tc_mma_f16_ts(leader, d, a + 16, bdesc + 4, idesc, 1u);
-            tc_mma_f16_ts(leader, d, a + 24, bdesc + 6, idesc, 1u);
-            accumulate = 1u;
-            a += 32;
-            bdesc += b_step;
+        tc_wait(p, &sh, &sh.a_full[sa], (uint32_t)((blk >> 1) & 1));
+        const uint32_t a = tmem + TC_A_COL + 128u * (uint32_t)sa;
+        uint64_t bdesc = bdesc0 + (uint64_t)(sb * p.bk) * b_step;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if ((k & (p.bk - 1)) == 0) {
+            tc_wait(p, &sh, &sh.b_full[sb], pb);
+            __syncwarp();
+            tc_fence_after();
           }
-          tc_commit_if(leader, &sh.b_empty[sb]);
-          if (++sb == p.b_stages) { sb = 0; pb ^= 1u; bdesc = bdesc0; }
+          tc_mma_f16_ts4(leader, d, a + 32 * k, bdesc, idesc, (uint32_t)(i | k));
+          bdesc += b_step;
+          if (((k + 1) & (p.bk - 1)) == 0) {
+            tc_commit_if(leader, &sh.b_empty[sb]);
+            if (++sb == p.b_stages) { sb = 0; pb ^= 1u; bdesc = bdesc0; }
+          }
         }
-        if (!ok) break;
         tc_commit_if(leader, &sh.a_empty[sa]);
       }
-      if (ok) tc_commit_if(leader, &sh.acc_full[buf]);
+      tc_commit_if(leader, &sh.acc_full[buf]);
     }
     // the block frees the tensor memory that MMAs in flight write: the epilogue waits for them too, but not after a give-up
     tc_commit_if(leader, &sh.drained);
     mbar_wait(&sh.drained, 0);
     __syncwarp();
-  } else if (warp == TC_WORKERS / 32 + 2) {
+  } else if (warp == 2) {
     // ---- activation producer ----
     if (lane == 0) {
       pdl_wait();
@@ -589,11 +715,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
       }
     }
     __syncwarp();
-  } else if (warp == TC_WORKERS / 32 + 1) {
+  } else if (warp == 1) {
     // ---- weight producer: eight lanes copy the block's eight cells (row groups past the image repeat its last one; the
     //      results of such rows are dropped) ----
-    const int nw = p.w_stages;
-    int blk = 0;
+    int blk = 0, stage = 0;
+    uint32_t par = 1;  // a fresh ring's stages count as empty
     bool ok = true;
     for (int u = 0; ok && tc_work(p, blockIdx.x, u, w); ++u) {
       const GemvSeg& sg = p.seg[w.seg];
@@ -602,10 +728,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
       const uint8_t* src = sg.img + ((size_t)group * p.nblk + w.b0) * cell;
 #pragma unroll 1
       for (int i = 0; i < w.nb; ++i, ++blk, src += cell) {
-        const int stage = blk % nw;
         void* bar = &sh.w_full[stage];
         if (lane == 0) {
-          ok = blk < nw || tc_wait(p, &sh, &sh.w_empty[stage], (uint32_t)((blk / nw - 1) & 1));
+          ok = blk < p.w_stages || tc_wait(p, &sh, &sh.w_empty[stage], par);
           if (ok) {
             mbar_expect_tx(bar, 8 * cell);
             *(volatile int*)&sh.w_issued = blk + 1;
@@ -614,71 +739,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
         ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
         if (!ok) break;
         if (lane < 8) bulk_g2s(Wbase + (size_t)stage * p.w_stage_bytes + (size_t)lane * cell, src, cell, bar);
+        if (++stage == p.w_stages) { stage = 0; par ^= 1u; }
       }
     }
     __syncwarp();
-  } else {
-    // ---- dequantising warps, then the epilogue: warp w holds TMEM lanes 32*(w & 3) .. +31 (= weight rows), the four warp
-    //      groups split the tokens ----
-    const int r = 32 * (warp & 3) + lane;
-    const int q_cols = p.NT / 4, c_begin = (warp >> 2) * q_cols;  // NT is a multiple of 32
-    int blk = 0;
-    for (int u = 0; tc_work(p, blockIdx.x, u, w); ++u) {
-      const int type = p.seg[w.seg].type;
-      if (type == T_Q4_K) tc_dequant_unit<T_Q4_K>(p, sh, Wbase, tmem, w, blk);
-      else if (type == T_Q6_K) tc_dequant_unit<T_Q6_K>(p, sh, Wbase, tmem, w, blk);
-      else tc_dequant_unit<T_Q8_0>(p, sh, Wbase, tmem, w, blk);
-      blk += w.nb;
-      const int buf = nbuf == 2 ? (u & 1) : 0, use = nbuf == 2 ? (u >> 1) : u;
-      if (u == 0) pdl_wait();
-      tc_wait(p, &sh, &sh.acc_full[buf], (uint32_t)(use & 1));
-      __syncwarp();
-      tc_fence_after();
-      const uint32_t acc = tmem + 128u * (uint32_t)buf + ((uint32_t)(32 * (warp & 3)) << 16);
-      const int c_end = min(c_begin + q_cols, p.T - w.t0);
-      const bool whole = w.c0 == w.c1;
-      float* part = p.ws + (whole ? 0 : (size_t)tc_slot(p, blockIdx.x, w.tile) * p.NT * TC_M) + r;
+  } else if (warp >= TC_SERVICE) {
+    // ---- dequantising warps, and the epilogue ----
+    const int group = (warp - TC_SERVICE) / TC_GROUP;
+    TcStand at{group, 0, 0u};
+    if (group && ++at.stage == p.w_stages) { at.stage = 0; at.par ^= 1u; }
+    int begin = 0;  // blocks of the units before
 #pragma unroll 1
-      for (int c0 = c_begin; c0 < c_end; c0 += 8) {
-        float v[8];
-        tc_ld8(acc + (uint32_t)c0, v);
-        if (whole) {
-          tc_finish8(p, w, w.row0 + r, w.t0 + c0, v);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) __stcg(part + (size_t)(c0 + j) * TC_M, v[j]);
+    for (int u = 0;; ++u) {
+      // The first block that each group has of this unit comes before the epilogue of the unit before, so that the MMAs go on as soon as an
+      // accumulator is free.
+      const bool more = tc_work(p, blockIdx.x, u, w);
+      const int type = more ? p.seg[w.seg].type : 0, nb = more ? w.nb : 0;
+#pragma unroll 1
+      for (int rest = 0; rest < 2; ++rest) {
+        const int end = begin + (rest ? nb : min(2, nb));
+        if (type == T_Q4_K) tc_dequant_to<T_Q4_K>(p, sh, Wbase, tmem, at, end);
+        else if (type == T_Q6_K) tc_dequant_to<T_Q6_K>(p, sh, Wbase, tmem, at, end);
+        else if (type == T_Q8_0) tc_dequant_to<T_Q8_0>(p, sh, Wbase, tmem, at, end);
+        if (rest == 0 && u > 0) {
+          tc_work(p, blockIdx.x, u - 1, w);
+          tc_epilogue(p, sh, tmem, w, u - 1, nbuf);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.acc_empty[buf]);
-      if (!whole) {
-        __threadfence();
-        tc_workers_sync();
-        if (tid == 0) {
-          sh.last = atomicAdd(&p.tickets[w.tile], 1) == w.c1 - w.c0;
-          if (sh.last) p.tickets[w.tile] = 0;
-          __threadfence();
-        }
-        tc_workers_sync();
-        const bool fin = sh.last != 0;
-        if (fin) {
-#pragma unroll 1
-          for (int c0 = c_begin; c0 < c_end; c0 += 8) {
-            float v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = 0.f;
-#pragma unroll 2
-            for (int c = w.c0; c <= w.c1; ++c) {
-              const float* src = p.ws + (size_t)tc_slot(p, c, w.tile) * p.NT * TC_M + r;
-#pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] += __ldcg(src + (size_t)(c0 + j) * TC_M);
-            }
-            tc_finish8(p, w, w.row0 + r, w.t0 + c0, v);
-          }
-        }
-        tc_workers_sync();  // sh.last is read before the next unit writes it
-      }
+      if (!more) break;
+      begin += nb;
     }
   }
   tc_fence_before();
@@ -689,7 +778,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     for (int s = max(0, sh.b_issued - p.b_stages); s < sh.b_issued; ++s) mbar_wait(&sh.b_full[s % p.b_stages], (uint32_t)((s / p.b_stages) & 1));
   }
   __syncthreads();
-  if (warp == 0) tc_dealloc(tmem, 512);
+  if (warp == 3) tc_dealloc(tmem, 512);
 }
 
 // x16[t][k] = fp16(x[t][k]) or, with norm weights, fp16(RMSNorm(x[t])[k]) (reference rmsnorm_batch_cpu,

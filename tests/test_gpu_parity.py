@@ -591,6 +591,25 @@ def test_batch_decode_grouped_query_attention_long_contexts(pkg, tiny_models, kv
 
 
 @pytest.mark.parametrize("kv", ["f32", "i8"])
+def test_prefill_batch_of_many_short_prompts(pkg, tiny_models, kv):
+    """40 prompts of 1 to 13 tokens in one call: more runs than a launch of prompt attention holds (32), runs of one token, a chunk's runs in
+    one grid. Logits against one call per sequence of the same tokens behind a neighbour that makes up the sixteen tokens of the
+    tensor-core path: columns of the products and rows of attention are their own. Tolerance as in the test below."""
+    kvd = pkg.KV_I8 if kv == "i8" else pkg.KV_F32
+    rng = np.random.default_rng(41)
+    prompts = [rng.integers(0, 512, 1 + 5 * i % 13).astype(np.int32) for i in range(40)]
+    filler = rng.integers(0, 512, 20).astype(np.int32)
+    a = pkg.Engine.from_gguf(tiny_models[1], max_seqs=41, kv_dtype=kvd)
+    b = pkg.Engine.from_gguf(tiny_models[1], max_seqs=41, kv_dtype=kvd)
+    got = a.prefill_batch(prompts, slots=list(range(40)))
+    for i in (0, 1, 2, 7, 31, 32, 33, 38, 39):
+        one = b.prefill_batch([filler, prompts[i]], slots=[40, i])[1]
+        assert np.abs(got[i] - one).max() <= (1e-4 if kv == "f32" else max(1e-4, 1.5e-2 * float(np.abs(one).max()))), i
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("kv", ["f32", "i8"])
 def test_prefill_batch_equals_one_call_per_sequence(pkg, tiny_models, kv):
     """Sequence-aware ingestion of ragged prompts in shared 512-token chunks (nine sequences, 860 tokens: two chunks, a
     prompt that straddles the chunk border, prompts shorter than a tile) against one b200_prefill call per sequence:

@@ -1,4 +1,4 @@
-// Prompt-ingestion attention: causal attention of a chunk of consecutive tokens of ONE sequence
+// Prompt-ingestion attention: causal attention of runs of consecutive tokens, each of one sequence,
 // against that sequence's KV cache (the chunk's own rows are already appended), on the fp16
 // tensor cores (mma.sync m16n8k16, FP32 accumulation).
 //
@@ -20,16 +20,23 @@
 
 namespace b200 {
 
+// Consecutive tokens of one sequence: rows row0 .. row0 + T - 1 of q and out, at positions start .. of KV slot `slot`.
+struct PrefillAttnRun {
+  int row0, T, slot, start;
+};
+constexpr int PFA_RUNS = 32;  // runs of a launch (short prompts ingested together: one launch each took 5 us a layer and prompt)
+
 struct PrefillAttnParams {
-  const float* q;  // [T][q_stride], after RoPE
+  const float* q;  // [rows][q_stride], after RoPE
   int q_stride;
   const void* k_cache;  // this layer's cache: [(slot*nkv + kvh)*max_ctx + pos][hd]
   const void* v_cache;
   const float* k_scale;  // [(slot*nkv + kvh)*max_ctx + pos] (INT8 cache only)
   const float* v_scale;
-  int slot, start, T;  // tokens occupy positions start .. start+T-1
+  PrefillAttnRun run[PFA_RUNS];
+  int nruns;
   int nq, nkv, max_ctx;
-  float* out;     // [T][out_stride], or
+  float* out;     // [rows][out_stride], or
   __half* out16;  // the same in fp16, the output projection's operand; one of the two
   int out_stride;
   float att_scale;
@@ -95,20 +102,27 @@ __global__ void __launch_bounds__(PFA_THREADS, 2) attn_prefill_kernel(const Pref
   unsigned char* raw = reinterpret_cast<unsigned char*>(vs_s + PFA_K);  // [2][K | V][PFA_K*HD] (INT8 cache)
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int q0 = blockIdx.x * PFA_Q, h = blockIdx.y;
+  // the run and its 64 queries; the last ones, which see most keys, first
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  int qt = gridDim.x - 1 - blockIdx.x, rn = 0;
+  while (rn + 1 < prm.nruns && qt >= (prm.run[rn].T + PFA_Q - 1) / PFA_Q) { qt -= (prm.run[rn].T + PFA_Q - 1) / PFA_Q; ++rn; }
+  const int T = prm.run[rn].T, start = prm.run[rn].start;
+  const size_t row0 = prm.run[rn].row0;
+  const int q0 = qt * PFA_Q, h = blockIdx.y;
   const int kvh = h / (prm.nq / prm.nkv);
-  const size_t crow0 = ((size_t)prm.slot * prm.nkv + kvh) * prm.max_ctx;
-  const int qend = min(q0 + PFA_Q, prm.T);       // queries of this CTA: q0 .. qend-1
-  const int kmax = prm.start + qend - 1;         // last key any of them sees
+  const size_t crow0 = ((size_t)prm.run[rn].slot * prm.nkv + kvh) * prm.max_ctx;
+  const int qend = min(q0 + PFA_Q, T);       // queries of this CTA: q0 .. qend-1
+  const int kmax = start + qend - 1;         // last key any of them sees
   const int nkt = kmax / PFA_K + 1;
 
   // this thread's two query rows and their Q fragments
   const int r0 = q0 + warp * 16 + g, r1 = r0 + 8;
-  const int qpos0 = prm.start + r0, qpos1 = prm.start + r1;
+  const int qpos0 = start + r0, qpos1 = start + r1;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t qa[KSTEPS][4];
   {
-    const float* qr0 = prm.q + (size_t)min(r0, prm.T - 1) * prm.q_stride + h * HD;
-    const float* qr1 = prm.q + (size_t)min(r1, prm.T - 1) * prm.q_stride + h * HD;
+    const float* qr0 = prm.q + (row0 + min(r0, T - 1)) * prm.q_stride + h * HD;
+    const float* qr1 = prm.q + (row0 + min(r1, T - 1)) * prm.q_stride + h * HD;
 #pragma unroll
     for (int ks = 0; ks < KSTEPS; ++ks) {
       const float2 a = *reinterpret_cast<const float2*>(qr0 + ks * 16 + 2 * t);
@@ -271,8 +285,8 @@ __global__ void __launch_bounds__(PFA_THREADS, 2) attn_prefill_kernel(const Pref
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
   const float inv0 = 1.0f / (l0 + 1e-9f), inv1 = 1.0f / (l1 + 1e-9f);  // softmax_vector_cpu (utils.cpp:675-698)
-  if (r0 < prm.T) {
-    const size_t at = (size_t)r0 * prm.out_stride + h * HD + 2 * t;
+  if (r0 < T) {
+    const size_t at = (row0 + r0) * prm.out_stride + h * HD + 2 * t;
     if (prm.out16) {
 #pragma unroll
       for (int i = 0; i < NT_O; ++i) *reinterpret_cast<uint32_t*>(prm.out16 + at + i * 8) = pfa_pack(o[i][0] * inv0, o[i][1] * inv0);
@@ -281,8 +295,8 @@ __global__ void __launch_bounds__(PFA_THREADS, 2) attn_prefill_kernel(const Pref
       for (int i = 0; i < NT_O; ++i) *reinterpret_cast<float2*>(prm.out + at + i * 8) = make_float2(o[i][0] * inv0, o[i][1] * inv0);
     }
   }
-  if (r1 < prm.T) {
-    const size_t at = (size_t)r1 * prm.out_stride + h * HD + 2 * t;
+  if (r1 < T) {
+    const size_t at = (row0 + r1) * prm.out_stride + h * HD + 2 * t;
     if (prm.out16) {
 #pragma unroll
       for (int i = 0; i < NT_O; ++i) *reinterpret_cast<uint32_t*>(prm.out16 + at + i * 8) = pfa_pack(o[i][2] * inv1, o[i][3] * inv1);

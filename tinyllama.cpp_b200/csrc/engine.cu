@@ -96,21 +96,6 @@ static bool prefill_attn_available(int hd) {
   return on && (hd == 64 || hd == 128);
 }
 
-static void launch_prefill_attention(const PrefillAttnParams& a, bool kv_i8, int hd, cudaStream_t st) {
-  const dim3 grid((a.T + PFA_Q - 1) / PFA_Q, a.nq);
-  const size_t smem = pfa_smem_bytes(kv_i8, hd);
-  if (hd == 128) {
-    if (kv_i8) attn_prefill_kernel<true, 128><<<grid, PFA_THREADS, smem, st>>>(a);
-    else attn_prefill_kernel<false, 128><<<grid, PFA_THREADS, smem, st>>>(a);
-  } else if (hd == 64) {
-    if (kv_i8) attn_prefill_kernel<true, 64><<<grid, PFA_THREADS, smem, st>>>(a);
-    else attn_prefill_kernel<false, 64><<<grid, PFA_THREADS, smem, st>>>(a);
-  } else {
-    throw std::runtime_error("prompt attention kernel: head_dim must be 64 or 128");
-  }
-  CK(cudaGetLastError());
-}
-
 // Batched decode of grouped-query models: one CTA per (sequence, KV head) on the tensor cores.
 // B200_GQA_ATTN=0 keeps the per-head decode kernel, =2 also uses this kernel when every query head
 // has its own KV head.
@@ -272,6 +257,23 @@ static void launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, si
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
   CK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
+static void launch_prefill_attention(bool pdl, const PrefillAttnParams& a, bool kv_i8, int hd, cudaStream_t st) {
+  int tiles = 0;
+  for (int r = 0; r < a.nruns; ++r) tiles += (a.run[r].T + PFA_Q - 1) / PFA_Q;
+  const dim3 grid(tiles, a.nq), block(PFA_THREADS);
+  const size_t smem = pfa_smem_bytes(kv_i8, hd);
+  if (hd == 128) launch_pdl(pdl, kv_i8 ? attn_prefill_kernel<true, 128> : attn_prefill_kernel<false, 128>, grid, block, smem, st, a);
+  else if (hd == 64) launch_pdl(pdl, kv_i8 ? attn_prefill_kernel<true, 64> : attn_prefill_kernel<false, 64>, grid, block, smem, st, a);
+  else throw std::runtime_error("prompt attention kernel: head_dim must be 64 or 128");
+}
+
+// New K / V rows of n tokens into the cache.
+static void launch_kv_append(const b200_engine* e, const float* kv_new, const int* positions, const int* slots, int n, const LayerW& w, cudaStream_t st) {
+  const dim3 grid(n, (e->nkv + KVA_WARPS * KVA_ROWS - 1) / (KVA_WARPS * KVA_ROWS), 2);
+  launch_pdl(e->use_pdl, kv_append_kernel, grid, dim3(32 * KVA_WARPS), 0, st, kv_new, 2 * e->KVD, positions, slots, e->nkv, e->hd, e->max_ctx,
+             e->desc.kv_dtype == B200_KV_I8 ? 1 : 0, w.k_cache, w.v_cache, w.k_scale, w.v_scale);
 }
 
 // Bytes the producer requests before the consumers hold their input vector (B200_GEMV_EARLY_KB, default 80).
@@ -586,9 +588,7 @@ static int packed_forward_step(b200_engine* e, int batch, int nsplit, cudaStream
     };
     if (use_tc && gqa_attn_available(e->hd, e->nq, e->nkv)) {
       const bool i8 = e->desc.kv_dtype == B200_KV_I8;
-      kv_append_kernel<<<dim3(batch, (e->nkv + KVA_WARPS - 1) / KVA_WARPS, 2), 32 * KVA_WARPS, 0, st>>>(e->d_kvnew, 2 * KVD, e->d_positions, e->d_slots, e->nkv, e->hd, e->max_ctx, i8 ? 1 : 0,
-                                                             w.k_cache, w.v_cache, w.k_scale, w.v_scale);
-      CK(cudaGetLastError());
+      launch_kv_append(e, e->d_kvnew, e->d_positions, e->d_slots, batch, w, st);
       GqaAttnParams a{};
       a.q = e->d_q; a.q_stride = e->Hq;
       a.k_cache = w.k_cache; a.v_cache = w.v_cache; a.k_scale = w.k_scale; a.v_scale = w.v_scale;
@@ -763,17 +763,17 @@ static void prefill_chunk(b200_engine* e, int T, const std::vector<int>& meta, c
       p.rope = e->rope; p.positions = d_pos; p.head_dim = e->hd; p.max_pos = e->desc.max_position_embeddings;
       launch_linear(e, p, T, st, true, nullptr, e->pf_x16);
     }
-    kv_append_kernel<<<dim3(T, (e->nkv + KVA_WARPS - 1) / KVA_WARPS, 2), 32 * KVA_WARPS, 0, st>>>(e->pf_kvnew, 2 * KVD, d_pos, d_slot, e->nkv, e->hd, e->max_ctx, i8 ? 1 : 0, w.k_cache,
-                                                        w.v_cache, w.k_scale, w.v_scale);
-    CK(cudaGetLastError());
+    launch_kv_append(e, e->pf_kvnew, d_pos, d_slot, T, w, st);
     if (prefill_attn_available(e->hd)) {
-      for (const PrefillRun& r : runs) {
-        PrefillAttnParams a{};
-        a.q = e->pf_q + (size_t)r.row0 * e->Hq; a.q_stride = e->Hq;
-        a.k_cache = w.k_cache; a.v_cache = w.v_cache; a.k_scale = w.k_scale; a.v_scale = w.v_scale;
-        a.slot = r.slot; a.start = r.start; a.T = r.len; a.nq = e->nq; a.nkv = e->nkv; a.max_ctx = e->max_ctx;
-        a.out16 = reinterpret_cast<__half*>(e->pf_attn) + (size_t)r.row0 * e->Hq; a.out_stride = e->Hq; a.att_scale = 1.0f / std::sqrt((float)e->hd);
-        launch_prefill_attention(a, i8, e->hd, st);
+      PrefillAttnParams a{};
+      a.q = e->pf_q; a.q_stride = e->Hq;
+      a.k_cache = w.k_cache; a.v_cache = w.v_cache; a.k_scale = w.k_scale; a.v_scale = w.v_scale;
+      a.nq = e->nq; a.nkv = e->nkv; a.max_ctx = e->max_ctx;
+      a.out16 = reinterpret_cast<__half*>(e->pf_attn); a.out_stride = e->Hq; a.att_scale = 1.0f / std::sqrt((float)e->hd);
+      for (size_t i = 0; i < runs.size(); i += PFA_RUNS) {
+        a.nruns = (int)std::min<size_t>(PFA_RUNS, runs.size() - i);
+        for (int r = 0; r < a.nruns; ++r) a.run[r] = {runs[i + r].row0, runs[i + r].len, runs[i + r].slot, runs[i + r].start};
+        launch_prefill_attention(e->use_pdl, a, i8, e->hd, st);
       }
     } else {
       AttnParams a{};

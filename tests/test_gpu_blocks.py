@@ -425,6 +425,27 @@ def test_batches_of_unequal_requests_match_each_alone(pkg, case, name, dtype, ba
         assert err(tail[i:i + 1], refs[i][-1:]) < limit
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("name", ["long", "piz_long"])
+def test_steps_over_long_rows(pkg, case, name, dtype):
+    """Decode steps of one to four sequences on rows of 2061 and 2603 elements: more than one piece of a vector per thread, sixteen warps along
+    a row, chunks that a warp has and its neighbour has not, a last chunk of a few elements."""
+    cfg = {"long": bm.config([bm.latent(q_rank=530, ff=2603), bm.wkv(heads=2, dim=20, ff=0)], width=2061, vocab=150),
+           "piz_long": bm.pizilix([bm.attention(ff=2603), bm.rglru(ff=0)], width=2061, vocab=150)}[name]
+    c = case(name, cfg=cfg)
+    eng = engine(pkg, c, dtype, max_seqs=4, max_ctx=16)
+    seqs = [bm.tokens(c.cfg, 4, seed=200 + i) for i in range(4)]
+    refs = [c.plain(s) for s in seqs]
+    limit = max(c.limit(dtype, s) for s in seqs)
+    for batch in (1, 2, 3, 4):
+        for k in range(4):
+            logits, amax = eng.decode([s[k] for s in seqs[:batch]], [k] * batch, slots=list(range(batch)))
+            assert np.array_equal(amax, logits.argmax(axis=1))
+            for i in range(batch):
+                assert err(logits[i][None], refs[i][k][None]) < limit, (batch, k, i)
+    eng.close()
+
+
 def test_batch_over_a_large_odd_vocabulary(pkg, case):
     """17 x 127217 logits: one value more than a whole number of pages in each of the eight pieces that they travel in. The caller's
     buffer holds NaN before the call."""

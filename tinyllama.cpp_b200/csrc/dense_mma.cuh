@@ -1,0 +1,352 @@
+// Matvec over bfloat16 weights for decode batches of the block models, on the tensor cores (mma.sync): the launches of dense_gemv.cuh, with its
+// prologue and epilogues, for engines that run in bfloat16.
+//
+// Weights are the 16 x 16 A operand, straight from global memory into the fragments' registers: lane (g, t) holds 16-byte piece t of
+// every 32-element chunk of rows g and g + 8, which feeds two MMAs whose k index is a permutation of the chunk, the same for both operands. The B
+// columns are the activations, FP32 values as the sum of P = 3 bfloat16 planes (24 bits: column P v + p is plane p of vector v), so that
+// products stay as exact as with FP32 activations; sums are FP32.
+//
+// Why: dense_gemv_kernel reads 32 bytes of activations from shared memory and issues 16 FMAs and 8 conversions for every 16 bytes of two weight
+// rows and every vector. Here a chunk of 1 KB costs a warp 2 loads, 2 shared loads and 4 MMAs for up to five vectors. Steps of the 2048-wide
+// models, us, one / two / three / four sequences: Nezolix 496 / 634 / 742 / 787 before, 444 / 512 / 681 / 702 now, Pizilix 405 / 504 / 596 /
+// 633 and 369 / 418 / 557 / 578. What bounds a launch now: its prologue (16000 cycles with both norms and four vectors, 6000 for an input that is
+// used as it is; about 1000 instructions a thread that every CTA repeats), then 1.8 us a task and SM (64 KB, 80 % of HBM's rate). One loop
+// for all passes, and the norm weights ahead of the wait, took as long. Batches of five to eight stay on the row path: with one bfloat16 plane for
+// eight vectors here a session of eight took 9.8 ms against 8.5, the prologue again.
+//
+// A CTA takes tasks of 16 rows; its 16 warps share a task's chunks out (WK of them along K, 16 / WK tasks at once, the more the shorter the
+// rows). A warp has two sets of four chunks (two with four vectors: registers), one on its way while the other is multiplied, the first two
+// requested before the launch waits for the previous kernel. The warps' sums meet in shared memory (two buffers, one barrier a task) and are added in a fixed order.
+#pragma once
+#include "dense_gemv.cuh"
+
+namespace b200 {
+
+constexpr size_t DMM_SMEM = 180 * 1024;  // dynamic: the activation image
+constexpr int DMM_U = 4;  // chunks of a warp in flight: 8 x 16 bytes per lane
+
+// bytes between the columns of the activation image: 64 modulo 128, so that the eight lanes of a 16-byte access phase (two columns x
+// four pieces) fall in distinct banks
+__host__ __device__ __forceinline__ int dmm_col_bytes(int K) { return ((pad8(K) >> 3) + 11) / 8 * 8 * 16 - 64; }
+__host__ __device__ __forceinline__ size_t dmm_smem_bytes(int K, int cols) { return (size_t)cols * dmm_col_bytes(K); }
+// warps along K: four chunks of 32 elements each at least
+__host__ __device__ __forceinline__ int dmm_warps_k(int K) {
+  const int chunks = (pad8(K) / 8 + 3) / 4;
+  int w = 1;
+  while (w < DGV_WARPS && 2 * w * DMM_U <= chunks) w *= 2;
+  return w;
+}
+
+__device__ __forceinline__ void dmm_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint4 ldg128_stream(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+template <int NB>
+__global__ void __launch_bounds__(DGV_THREADS, 1) dense_mma_kernel(const DgvParams p, int wk) {
+  constexpr int P = 3, NC = NB * P, NG = (NC + 7) / 8, U = NB == 4 ? DMM_U / 2 : DMM_U;
+  extern __shared__ __align__(128) uint8_t dmm_x[];  // [NC columns][dmm_col_bytes]
+  __shared__ float red[DGV_WARPS * NB], fac[NB];
+  __shared__ __align__(16) float part[2][DGV_WARPS][16][8 * NG];
+  __shared__ float best_v[DGV_WARPS][NB];
+  __shared__ int best_i[DGV_WARPS][NB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int K = p.K, kc = pad8(K) >> 3, nch = (kc + 3) >> 2, b0 = blockIdx.y * NB;
+  const int kw = warp & (wk - 1), rg = warp / wk, RG = DGV_WARPS / wk;
+  pdl_launch_dependents();
+
+  // ---- tasks: groups of 16 matrix rows (eight outputs of a gated product) ----
+  const int seg_fixed = p.ctas_per_seg ? (int)blockIdx.x / p.ctas_per_seg : -1;
+  auto tasks_of = [&](int s) { return act_is_glu(p.seg[s].act) ? (p.seg[s].rows + 7) >> 3 : (p.seg[s].rows + 15) >> 4; };
+  int ntasks = 0, task, stride;
+  if (seg_fixed >= 0) {
+    ntasks = tasks_of(seg_fixed);
+    task = (blockIdx.x - seg_fixed * p.ctas_per_seg) * RG;
+    stride = p.ctas_per_seg * RG;
+  } else {
+    for (int s = 0; s < p.nseg; ++s) ntasks += tasks_of(s);
+    task = blockIdx.x * RG;
+    stride = gridDim.x * RG;
+  }
+  auto locate = [&](int n, int& seg) {  // task n: its segment; returns its number there
+    if (seg_fixed >= 0) { seg = seg_fixed; return n; }
+    seg = 0;
+    while (seg + 1 < p.nseg && n >= tasks_of(seg)) { n -= tasks_of(seg); ++seg; }
+    return n;
+  };
+  // this lane's two weight rows of a task, at its first piece (rows beyond the matrix repeat the last one; their sums are dropped)
+  const uint4 *w0 = nullptr, *w1 = nullptr;
+  auto rows_of = [&](int n) {
+    int seg;
+    const int i = locate(n, seg);
+    const DgvSeg& sg = p.seg[seg];
+    int64_t a, b;
+    if (act_is_glu(sg.act)) {
+      const int r = min(8 * i + g, sg.rows - 1);
+      a = glu_row(r, 0);
+      b = glu_row(r, 1);
+    } else {
+      a = min(16 * i + g, sg.rows - 1);
+      b = min(16 * i + 8 + g, sg.rows - 1);
+    }
+    w0 = reinterpret_cast<const uint4*>(sg.w) + a * kc;
+    w1 = reinterpret_cast<const uint4*>(sg.w) + b * kc;
+  };
+  // Two sets of four chunks: while one is multiplied the other is on its way, and a set is requested again as soon as it has been used.
+  uint4 sa[2][U], sb[2][U];
+  const int per = (nch + wk - 1) / wk;  // chunks of a warp
+  int next = task + rg, next_k = 0;     // what is requested next
+  auto request = [&](uint4 (&a)[U], uint4 (&b)[U]) {
+    if (next >= ntasks) return;
+    if (next_k == 0) rows_of(next);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = 4 * (kw + (next_k + u) * wk) + t;
+      const bool ok = c < kc;
+      a[u] = ok ? ldg128_stream(w0 + c) : make_uint4(0, 0, 0, 0);
+      b[u] = ok ? ldg128_stream(w1 + c) : make_uint4(0, 0, 0, 0);
+    }
+    next_k += U;
+    if (next_k >= per) { next_k = 0; next += stride; }
+  };
+  request(sa[0], sb[0]);
+  request(sa[1], sb[1]);
+  pdl_wait();
+
+  // ---- prologue (dense_gemv.cuh): piece j of all vectors is requested together, rows of up to 2048 elements stay in registers
+  //      between the passes, longer ones come from L1 again ----
+  const int n4 = 2 * kc, col_bytes = dmm_col_bytes(K);
+  const float* mu = seg_fixed >= 0 ? p.seg[seg_fixed].mu : nullptr;
+  float4 keep[NB], kadd[NB];
+  float ss[NB], sx[NB];
+  auto piece = [&](const float* base, int j, float4 (&v)[NB]) {
+#pragma unroll
+    for (int n = 0; n < NB; ++n) v[n] = b0 + n < p.batch ? ld4_masked(base + (size_t)(b0 + n) * p.x_stride, 4 * j, K) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto squares = [&](const float4 (&v)[NB], float (&s)[NB]) {
+#pragma unroll
+    for (int n = 0; n < NB; ++n) s[n] += v[n].x * v[n].x + v[n].y * v[n].y + v[n].z * v[n].z + v[n].w * v[n].w;
+  };
+  // 1 / rms of every vector: a warp finishes one, all read it
+  auto inverse = [&](float (&s)[NB]) {
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+      s[n] = warp_sum(s[n]);
+      if (lane == 0) red[n * DGV_WARPS + warp] = s[n];
+    }
+    __syncthreads();
+    if (warp < NB) {
+      float r = red[warp * DGV_WARPS + (lane & (DGV_WARPS - 1))];
+#pragma unroll
+      for (int o = 1; o < DGV_WARPS; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+      if (lane == 0) fac[warp] = 1.0f / sqrtf(r / (float)K + p.eps);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < NB; ++n) s[n] = fac[n];
+  };
+  // the residual stream with what is pending added; v, a: piece j of the stream and of the pending output
+  auto stream = [&](int j, float4 (&v)[NB], const float4 (&a)[NB]) {
+    if (!p.add) return;
+    const float4 w = p.add_w ? ld4_masked(p.add_w, 4 * j, K) : make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+      const float f = p.add_w ? ss[n] : 1.f;
+      v[n].x += a[n].x * f * w.x; v[n].y += a[n].y * f * w.y; v[n].z += a[n].z * f * w.z; v[n].w += a[n].w * f * w.w;
+    }
+    if (p.add2) {
+      float4 e[NB];
+      piece(p.add2, j, e);
+#pragma unroll
+      for (int n = 0; n < NB; ++n) { v[n].x += e[n].x; v[n].y += e[n].y; v[n].z += e[n].z; v[n].w += e[n].w; }
+    }
+  };
+  if (tid < n4) {
+    piece(p.x, tid, keep);
+    if (p.add) piece(p.add, tid, kadd);
+  }
+  if (p.add && p.add_w) {
+#pragma unroll
+    for (int n = 0; n < NB; ++n) ss[n] = 0.f;
+    if (tid < n4) squares(kadd, ss);
+#pragma unroll 1
+    for (int j = tid + DGV_THREADS; j < n4; j += DGV_THREADS) {
+      float4 a[NB];
+      piece(p.add, j, a);
+      squares(a, ss);
+    }
+    inverse(ss);
+  }
+  if (tid < n4) stream(tid, keep, kadd);
+  if (p.norm_w) {
+#pragma unroll
+    for (int n = 0; n < NB; ++n) sx[n] = 0.f;
+    if (tid < n4) squares(keep, sx);
+#pragma unroll 1
+    for (int j = tid + DGV_THREADS; j < n4; j += DGV_THREADS) {
+      float4 v[NB], a[NB];
+      piece(p.x, j, v);
+      if (p.add) piece(p.add, j, a);
+      stream(j, v, a);
+      squares(v, sx);
+    }
+    inverse(sx);
+  }
+#pragma unroll 1
+  for (int j = tid; j < n4; j += DGV_THREADS) {
+    if (j != tid) {
+      piece(p.x, j, keep);
+      if (p.add) piece(p.add, j, kadd);
+      stream(j, keep, kadd);
+    }
+    const float4 w = p.norm_w ? ld4_masked(p.norm_w, 4 * j, K) : make_float4(1.f, 1.f, 1.f, 1.f);
+    const float4 m4 = p.shift ? ld4_masked(mu, 4 * j, K) : w;
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+      float4 v = keep[n];
+      const bool there = b0 + n < p.batch;
+      if (p.add && blockIdx.x == 0 && there) *reinterpret_cast<float4*>(p.x_out + (size_t)(b0 + n) * p.x_stride + 4 * j) = v;
+      if (p.norm_w) {
+        const float f = sx[n];
+        v.x *= f * w.x; v.y *= f * w.y; v.z *= f * w.z; v.w *= f * w.w;
+        if (p.shift && there) {
+          const int pos = p.positions[b0 + n];
+          float* hist = p.shift + (size_t)p.slots[b0 + n] * 2 * p.shift_stride;
+          const float4 o = pos > 0 ? ld4_masked(hist + (size_t)(pos & 1) * p.shift_stride, 4 * j, K) : make_float4(0.f, 0.f, 0.f, 0.f);
+          if (blockIdx.x == 0) *reinterpret_cast<float4*>(hist + (size_t)((pos + 1) & 1) * p.shift_stride + 4 * j) = v;
+          v.x += (o.x - v.x) * m4.x; v.y += (o.y - v.y) * m4.y; v.z += (o.z - v.z) * m4.z; v.w += (o.w - v.w) * m4.w;
+        }
+      }
+      if (!there) v = make_float4(0.f, 0.f, 0.f, 0.f);
+      uint8_t* col = dmm_x + (size_t)n * P * col_bytes + 8 * j;
+#pragma unroll
+      for (int q = 0; q < P; ++q) {  // the leading bfloat16 of what is left
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+        *reinterpret_cast<uint2*>(col + (size_t)q * col_bytes) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        if (q + 1 < P) {
+          v.x -= __bfloat162float(lo.x); v.y -= __bfloat162float(lo.y);
+          v.z -= __bfloat162float(hi.x); v.w -= __bfloat162float(hi.y);
+        }
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- products ----
+  const uint8_t* bcol[NG];  // this lane's piece of the first chunk of column g of each group; nullptr: a column that carries nothing
+#pragma unroll
+  for (int i = 0; i < NG; ++i) bcol[i] = 8 * i + g < NC ? dmm_x + (size_t)(8 * i + g) * col_bytes + 16 * t : nullptr;
+  float bv[NB];
+  int bi[NB];
+#pragma unroll
+  for (int n = 0; n < NB; ++n) { bv[n] = -INFINITY; bi[n] = 0x7fffffff; }
+  int turn = 0;
+  bool odd = false;
+#pragma unroll 1
+  for (; task < ntasks; task += stride, ++turn) {
+    const bool mine = task + rg < ntasks;
+    float c[NG][4];
+#pragma unroll
+    for (int i = 0; i < NG; ++i) c[i][0] = c[i][1] = c[i][2] = c[i][3] = 0.f;
+    auto multiply = [&](const uint4 (&a)[U], const uint4 (&b)[U], int k) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int ch = kw + (k + u) * wk;
+        const bool in = 4 * ch + t < kc;  // pieces beyond the row: nothing in the image
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+          const uint4 x = bcol[i] && in ? *reinterpret_cast<const uint4*>(bcol[i] + 64 * ch) : make_uint4(0, 0, 0, 0);
+          dmm_mma(c[i], a[u].x, b[u].x, a[u].y, b[u].y, x.x, x.y);
+          dmm_mma(c[i], a[u].z, b[u].z, a[u].w, b[u].w, x.z, x.w);
+        }
+      }
+    };
+    if (mine) {
+#pragma unroll 1
+      for (int k = 0; k < per; k += U, odd = !odd) {
+        if (odd) {
+          multiply(sa[1], sb[1], k);
+          request(sa[1], sb[1]);
+        } else {
+          multiply(sa[0], sb[0], k);
+          request(sa[0], sb[0]);
+        }
+      }
+    }
+    float(*mypart)[8 * NG] = part[turn & 1][warp];
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+      *reinterpret_cast<float2*>(&mypart[g][8 * i + 2 * t]) = make_float2(c[i][0], c[i][1]);
+      *reinterpret_cast<float2*>(&mypart[g + 8][8 * i + 2 * t]) = make_float2(c[i][2], c[i][3]);
+    }
+    __syncthreads();  // by the next one all have read this buffer
+    // ---- 16 rows x NB vectors of each of the RG tasks: sums over warps and planes, then the epilogue; other warps each turn ----
+#pragma unroll 1
+    for (int base = (tid - lane + 96 * turn) & (DGV_THREADS - 1); base < RG * 16 * NB; base += DGV_THREADS) {
+      const int idx = base + lane, r = idx & 15, v = (idx >> 4) % NB, q = (idx >> 4) / NB, b = b0 + v, n = task + q;
+      const bool there = q < RG && n < ntasks;
+      float sum = 0.f;
+      if (there)
+        for (int w = 0; w < wk; ++w) {
+          const float* s = &part[turn & 1][q * wk + w][r][v * P];
+#pragma unroll
+          for (int i = P - 1; i >= 0; --i) sum += s[i];
+        }
+      int seg = 0, i = 0;
+      if (there) i = locate(n, seg);
+      const DgvSeg& sg = p.seg[seg];
+      const bool glu = act_is_glu(sg.act);
+      const float up = __shfl_down_sync(0xffffffffu, sum, 8);
+      const int row = glu ? 8 * i + r : 16 * i + r;
+      if (there && b < p.batch && row < sg.rows && !(glu && r >= 8)) {
+        if (glu) {
+          sg.y[(size_t)b * sg.y_stride + row] = glu_act(sg.act, sum, up);
+        } else {
+          float o = dense_act(sg.act, sg.bias ? sum + sg.bias[row] : sum, sg.arg);
+          if (p.pen_counts) {
+            const int times = p.pen_counts[(size_t)b * p.pen_stride + row];
+            const float pen = *p.pen_value;
+            for (int k = 0; k < times; ++k) o = o > 0.f ? o / pen : o * pen;
+          }
+          sg.y[(size_t)b * sg.y_stride + row] = o;
+          if (p.amax_val) {
+#pragma unroll
+            for (int k = 0; k < NB; ++k)
+              if (k == v && (o > bv[k] || (o == bv[k] && row < bi[k]))) { bv[k] = o; bi[k] = row; }
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+  if (p.amax_val) {
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv[n], o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi[n], o);
+        if (ov > bv[n] || (ov == bv[n] && oi < bi[n])) { bv[n] = ov; bi[n] = oi; }
+      }
+      if (lane == 0) { best_v[warp][n] = bv[n]; best_i[warp][n] = bi[n]; }
+    }
+    __syncthreads();
+    if (tid < NB && b0 + tid < p.batch) {
+      float v = best_v[0][tid];
+      int i = best_i[0][tid];
+      for (int w = 1; w < DGV_WARPS; ++w)
+        if (best_v[w][tid] > v || (best_v[w][tid] == v && best_i[w][tid] < i)) { v = best_v[w][tid]; i = best_i[w][tid]; }
+      p.amax_val[(size_t)(b0 + tid) * gridDim.x + blockIdx.x] = v;
+      p.amax_idx[(size_t)(b0 + tid) * gridDim.x + blockIdx.x] = i;
+    }
+  }
+}
+
+}  // namespace b200

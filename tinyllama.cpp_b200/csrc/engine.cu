@@ -15,6 +15,7 @@
 #include "attn_stream.cuh"
 #include "block_model.h"
 #include "dense_gemm.cuh"
+#include "dense_mma.cuh"
 #include "dequant.cuh"
 #include "gemv.cuh"
 #include "gemv_batch.cuh"

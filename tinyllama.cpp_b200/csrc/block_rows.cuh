@@ -53,6 +53,8 @@ __global__ void __launch_bounds__(ROW_THREADS) norm_rows_kernel(const NormRowsPa
   extern __shared__ __align__(16) float row_s[];
   __shared__ float red[ROW_THREADS / 32];
   const int tid = threadIdx.x, n4 = pad8(p.W) >> 2;
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t src = p.gather ? (size_t)p.gather[blockIdx.x] : blockIdx.x;
   float* xr = p.x + src * p.x_stride;
   float4* s4 = reinterpret_cast<float4*>(row_s);

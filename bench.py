@@ -454,7 +454,7 @@ def main():
     vocab = eng.vocab
     pr = prompts(batch, prompt_len, vocab)
     t_prefill = time.perf_counter()
-    if batch > 1:  # all prompts in one sequence-aware call (shared 512-token chunks)
+    if batch > 1:  # all prompts in one sequence-aware call (shared chunks)
         first = [int(v.argmax()) for v in eng.prefill_batch(pr)]
     else:
         first = [int(eng.prefill(pr[0], slot=0).argmax())]

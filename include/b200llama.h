@@ -98,7 +98,7 @@ int b200_prefill(b200_engine* e, int seq_slot, const int32_t* token_ids, int n, 
 /* Sequence-aware prompt ingestion of several sequences in one call (the batch prefill of
  * TinyLlamaSession::generate_batch, api.cpp:1144-1421, with attention_batch_cpu_sequence_aware,
  * cpu_attention.cpp:203-325): the prompts are laid end to end (token_ids holds lens[0] + lens[1] + ... ids) and cut
- * into chunks of 512 tokens, so that short prompts share a chunk and its weight traffic; every token carries its own
+ * into chunks of up to 2048 tokens (512 under tensor parallelism), so that short prompts share a chunk and its weight traffic; every token carries its own
  * position and KV slot, and each token attends only to its own sequence's rows. Always the tensor-core path.
  * Sequence s occupies positions start_pos[s] .. start_pos[s]+lens[s]-1 of slot slots[s] (slots distinct).
  * host_logits_last [n_seqs][vocab] (logits after each prompt's last token) may be NULL. Same kernels and the same
@@ -111,7 +111,8 @@ int b200_prefill_rows(b200_engine* e, int seq_slot, const int32_t* token_ids, in
                       float* host_logits);
 /* The chunk plan b200_prefill_batch follows for prompts of these lengths (host arithmetic only, no GPU needed): one
  * record per run of tokens, out[i] = {chunk, first row in the chunk, tokens, position of the first token, index of the
- * sequence whose prompt ends with this run or -1}. chunk = tokens per chunk (the engine uses 512). */
+ * sequence whose prompt ends with this run or -1}. chunk = tokens per chunk (the engine uses 2048, or less
+ * where its buffers find no room). */
 int b200_prefill_plan(int n_seqs, const int32_t* lens, int chunk, int32_t* out /* [max_runs][5] */, int max_runs, int* n_runs);
 
 /* One decode step for `batch` independent sequences: forward_device_batch_generation

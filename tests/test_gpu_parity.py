@@ -591,6 +591,26 @@ def test_batch_decode_grouped_query_attention_long_contexts(pkg, tiny_models, kv
 
 
 @pytest.mark.parametrize("kv", ["f32", "i8"])
+def test_prefill_batch_over_chunks(pkg, tiny_models, kv):
+    """20 prompts, 2305 tokens: more than a chunk of 2048, whose border falls inside a prompt. Logits of the last prompts against one call
+    each (tolerance as in the tests around)."""
+    kvd = pkg.KV_I8 if kv == "i8" else pkg.KV_F32
+    rng = np.random.default_rng(43)
+    prompts = [rng.integers(0, 512, 127 - 3 * i % 13 - 3 * (i % 5)).astype(np.int32) for i in range(20)]
+    ends = np.cumsum([len(p) for p in prompts])
+    cut = int(np.searchsorted(ends, 2048))
+    assert ends[-1] > 2048 and ends[cut] != 2048 and cut < 19
+    a = pkg.Engine.from_gguf(tiny_models[1], max_seqs=20, kv_dtype=kvd)
+    b = pkg.Engine.from_gguf(tiny_models[1], max_seqs=20, kv_dtype=kvd)
+    got = a.prefill_batch(prompts, slots=list(range(20)))
+    for i in (0, cut - 1, cut, cut + 1, 19):
+        one = b.prefill(prompts[i], slot=i)
+        assert np.abs(got[i] - one).max() <= (1e-4 if kv == "f32" else max(1e-4, 1.5e-2 * float(np.abs(one).max()))), i
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("kv", ["f32", "i8"])
 def test_prefill_batch_of_many_short_prompts(pkg, tiny_models, kv):
     """40 prompts of 1 to 13 tokens in one call: more runs than a launch of prompt attention holds (32), runs of one token, a chunk's runs in
     one grid. Logits against one call per sequence of the same tokens behind a neighbour that makes up the sixteen tokens of the

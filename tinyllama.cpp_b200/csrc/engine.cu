@@ -710,11 +710,21 @@ static int enqueue_step(b200_engine* e, int batch, int nsplit, cudaStream_t st, 
 // the fp16 tensor cores; head sizes other than 64 / 128: the decode-attention kernel per token) runs
 // over the cache rows up to and including each token's own position (causal). Only the last token's logits are
 // computed (the reference computes all rows and keeps the last, model.cpp:1094-1156).
-constexpr int PF_CHUNK = 512;
+// Tokens of a chunk: every chunk reads all weights, starts 4 matmuls a layer and cuts their last waves, so as many as the buffers find room
+// for. ms, chunks of 512 / 1024 / 2048: seven 1.1B prompts (1700 tokens) 10.4 / 7.25 / 5.42, a 7B prompt of 1024 tokens 20.6 / 17.2.
+// 512 under tensor parallelism, where all ranks have to choose alike.
+constexpr int PF_CHUNK = 2048, PF_CHUNK_SMALL = 512;
 
 static void ensure_prefill_buffers(b200_engine* e) {
   if (e->pf_cap) return;
-  const int T = PF_CHUNK;
+  int T = PF_CHUNK_SMALL;
+  if (e->tp_size == 1) {
+    size_t free = 0, total = 0;
+    CK(cudaMemGetInfo(&free, &total));
+    // the buffers below (partial results only of head sizes without prompt attention: up to 32 splits a head): at most a quarter of what is free
+    const size_t token = (size_t)12 * e->H + 8 * e->KVD + 4 * e->F + 2 * std::max(e->H, e->F) + 16 * e->nq * (e->hd < 64 ? 32 * (e->hd + 2) : e->hd + 2);
+    while (T < PF_CHUNK && free / 4 > 2 * T * token) T *= 2;
+  }
   e->pf_ints = dev_alloc<int>(e, (size_t)3 * T);
   e->pf_h = dev_alloc<float>(e, (size_t)T * e->H);
   e->pf_q = dev_alloc<float>(e, (size_t)T * e->H);
@@ -732,7 +742,7 @@ static void ensure_prefill_buffers(b200_engine* e) {
   e->pf_cap = T;
 }
 
-// One chunk of T <= PF_CHUNK prompt tokens, possibly of several sequences (sequence-aware: every token carries its
+// One chunk of T <= pf_cap prompt tokens, possibly of several sequences (sequence-aware: every token carries its
 // own position and KV slot through the RoPE epilogue and the cache append, and attention runs per run of tokens,
 // each over its own sequence's cache rows; reference api.cpp:1144-1421 / cpu_attention.cpp:203-325).
 // meta = token ids | positions | slots, T each. After the layers, the logits of the wanted rows are computed and copied
@@ -851,7 +861,8 @@ static void prefill_sequences(b200_engine* e, int n_seqs, const int32_t* slots, 
                               float* host_logits, const int32_t* want = nullptr, int n_want = 0) {
   std::vector<PrefillRun> all;
   std::vector<int> chunk_of;
-  plan_prefill_runs(n_seqs, slots, lens, start_pos, e->blocks ? e->blocks->chunk : PF_CHUNK, all, chunk_of);
+  if (!e->blocks) ensure_prefill_buffers(e);
+  plan_prefill_runs(n_seqs, slots, lens, start_pos, e->blocks ? e->blocks->chunk : e->pf_cap, all, chunk_of);
   std::vector<size_t> seq_off(n_seqs + 1, 0);
   for (int s = 0; s < n_seqs; ++s) seq_off[s + 1] = seq_off[s] + (size_t)lens[s];
   // which sequence a run belongs to: runs come in sequence order, a new sequence starts when the previous one's last run ended
